@@ -202,25 +202,43 @@ __global__ void interleave_keyed_kernel(const int *__restrict__ col, const unsig
 // One 32-byte tile per vertex (layout in mlmq_queue.cuh): up to TILE_ARCS
 // arcs inline, unused slots with dst -1; a vertex of higher degree holds
 // {TILE_CSR, first arc, degree} instead.
+// seen[0], seen[1]: of each vertex's first TILE_ARCS arcs, those that leave its
+// block of `block` consecutive vertices, and all.
 __global__ void tile_kernel(const int *__restrict__ row, const int2 *__restrict__ arcs,
-                            int4 *tiles, int n) {
+                            int4 *tiles, int n, unsigned block, unsigned *seen) {
+    unsigned away = 0, all = 0;
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         const int beg = row[v], deg = row[v + 1] - beg;
         int t[8] = {-1, 0, -1, 0, -1, 0, -1, 0};
+        const unsigned home = (unsigned)v / block;
+        for (int i = 0; i < min(deg, TILE_ARCS); i++) {
+            const int2 a = arcs[beg + i];
+            t[2 * i] = a.x;
+            t[2 * i + 1] = a.y;
+            away += (unsigned)a.x / block != home;
+            all++;
+        }
         if (deg > TILE_ARCS) {
             t[0] = TILE_CSR;
             t[1] = beg;
             t[2] = deg;
-        } else {
-            for (int i = 0; i < deg; i++) {
-                const int2 a = arcs[beg + i];
-                t[2 * i] = a.x;
-                t[2 * i + 1] = a.y;
-            }
+            t[3] = t[5] = t[7] = 0;
+            t[4] = t[6] = -1;
         }
         tiles[2 * (size_t)v] = make_int4(t[0], t[1], t[2], t[3]);
         tiles[2 * (size_t)v + 1] = make_int4(t[4], t[5], t[6], t[7]);
     }
+    __shared__ unsigned sums[2];
+    if (threadIdx.x < 2) sums[threadIdx.x] = 0u;
+    __syncthreads();
+    away = __reduce_add_sync(FULL, away);
+    all = __reduce_add_sync(FULL, all);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(sums, away);
+        atomicAdd(sums + 1, all);
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) atomicAdd(seen + threadIdx.x, sums[threadIdx.x]);
 }
 
 // Wide tiles from the 32-byte ones: a vertex of at most TILE_ARCS_WIDE arcs
@@ -549,7 +567,7 @@ struct ArcRange {
 // one part of the graph while the next is still being copied (R-MAT-22
 // upload 21.4 -> 14.7 ms, 9.8 ms of it the PCIe copy).
 int build_arcs(int n, int64_t m, const int *d_row, const int *d_col, const int *d_w,
-               const std::vector<ArcRange> &ranges, int2 *arcs) {
+               const std::vector<ArcRange> &ranges, int2 *arcs, int *max_degree) {
     int vbits = 1;
     while (vbits < 31 && ((n - 1) >> vbits) != 0) vbits++;
     int64_t max_arcs = 0;
@@ -573,6 +591,7 @@ int build_arcs(int n, int64_t m, const int *d_row, const int *d_col, const int *
         }
         if (!rc) rc = cuda_fail(cudaMemcpy(maxes, d_max, sizeof(maxes), cudaMemcpyDeviceToHost),
                                 "D2H max");
+        *max_degree = std::max(*max_degree, maxes[0]);
         const int cnt = (int)(r.a1 - r.a0);
         size_t need = 0;
         if (!rc && maxes[0] > SPLIT_MIN) {
@@ -661,7 +680,7 @@ int wrap_device(int n, int64_t m, const int *d_row, const int *d_col, const int 
     // graph can be built while a server kernel runs).
     int rc = cuda_fail(cudaGetDevice(&g->device), "cudaGetDevice");
     if (!rc) rc = dev_alloc(&g->d_arcs, sizeof(int2) * (size_t)(m > 0 ? m : 1), 0, "alloc(arcs)");
-    if (!rc && m > 0) rc = build_arcs(n, m, d_row, d_col, d_w, ranges, g->d_arcs);
+    if (!rc && m > 0) rc = build_arcs(n, m, d_row, d_col, d_w, ranges, g->d_arcs, &g->max_degree);
     // Heavy vertices (more than SPLIT_MIN arcs) are found on the device; at
     // most m / (SPLIT_MIN + 1) exist.  Their pieces are laid out on the host
     // in vertex order.
@@ -714,11 +733,22 @@ int wrap_device(int n, int64_t m, const int *d_row, const int *d_col, const int 
         g->pieces += np;
     }
     if (!rc) rc = dev_alloc(&g->d_tiles, 2 * sizeof(int4) * (size_t)g->slots(), 0, "alloc(tiles)");
+    // How far the vertex numbering keeps neighbours together, for the blocks
+    // that the vertex-owner kernel would use.
+    unsigned *d_seen = nullptr, seen[2] = {0, 0};
+    int sms = 0, ctas = 0;
+    if (!rc) rc = device_sm_count(&sms);
+    if (!rc) rc = dev_alloc(&d_seen, 2 * sizeof(unsigned), 0, "alloc(locality)");
+    if (!rc) rc = cuda_fail(cudaMemsetAsync(d_seen, 0, 2 * sizeof(unsigned), 0), "locality");
     if (!rc) {
         int blocks = (int)std::min<int64_t>(((int64_t)n + 255) / 256, 148 * 16);
-        tile_kernel<<<blocks, 256>>>(d_row, g->d_arcs, g->d_tiles, n);
+        tile_kernel<<<blocks, 256>>>(d_row, g->d_arcs, g->d_tiles, n,
+                                     (unsigned)std::max(1, owner_block(n, sms, &ctas)), d_seen);
         rc = cuda_fail(cudaGetLastError(), "tile launch");
     }
+    if (!rc) rc = cuda_fail(cudaMemcpy(seen, d_seen, sizeof(seen), cudaMemcpyDeviceToHost), "D2H locality");
+    if (seen[1]) g->away = (float)seen[0] / (float)seen[1];
+    dev_free(d_seen, 0);
     if (!rc && g->pieces > 0) {
         rc = cuda_fail(cudaMemcpy(g->d_tiles + 2 * (size_t)n, piece_tiles.data(),
                                   sizeof(int4) * piece_tiles.size(), cudaMemcpyHostToDevice),
@@ -925,6 +955,30 @@ extern "C" int mlmq_solver_create(const mlmq_graph *g, const mlmq_config *cfg_in
         mlmq_solver_destroy(s);
         return rc;
     }
+    // Vertices in a local order, none of many arcs, an SLF queue without the
+    // split or synchronised buckets: the vertex-owner kernel.  Its wavefront
+    // hops inside an SM; with many arcs between blocks it would send messages
+    // instead, and a vertex of many arcs would hold up its CTA's ticks.  Above
+    // OWNER_MAX_N vertices its longer lists and tiles from HBM take as long as
+    // the asynchronous kernel's hops (3M points 6.2 ms on both).
+    constexpr int OWNER_MAX_N = 3 << 20, OWNER_MAX_DEGREE = 32;
+    int owner_ctas = 0;
+    if (cfg.queue_type == MLMQ_L1SLF_L2DQ && !cfg.light_heavy && !cfg.bucket_sync &&
+        g->n <= OWNER_MAX_N && g->max_degree <= OWNER_MAX_DEGREE && g->away <= 0.125f) {
+        const int block = owner_block(g->n, sms, &owner_ctas);
+        if (block && (cfg.work_blocks == 0 || owner_ctas <= cfg.work_blocks)) s->owner_block = block;
+    }
+    if (s->owner_block) {
+        rc = cuda_fail(owner_prepare(), "owner shared memory");
+        // Vertices of more arcs than a 32-byte tile holds: 64-byte tiles, which
+        // save them a dependent load.
+        if (!rc && cfg.vertex_tiles == 1 && g->max_degree > TILE_ARCS)
+            rc = graph_tiles(g, 2, &s->tiles, &s->tile_stride);
+        if (rc) {
+            mlmq_solver_destroy(s);
+            return rc;
+        }
+    }
     s->l3_log = cfg.l3_cap_log2 ? cfg.l3_cap_log2 : l3_ring_log2(s->nids, g->m);
     s->workers = cfg.warps_per_block;
     int bps = 0;
@@ -934,6 +988,7 @@ extern "C" int mlmq_solver_create(const mlmq_graph *g, const mlmq_config *cfg_in
         const int maxgrid = bps * sms;
         s->grid = cfg.work_blocks > 0 ? std::min(cfg.work_blocks, maxgrid) : sms;
         if (s->grid > maxgrid) s->grid = maxgrid;
+        if (s->owner_block) s->grid = owner_ctas;
     }
     const size_t l2_bytes = sizeof(unsigned long long) * ((size_t)(cfg.bucket_num + 1) << s->l2_log);
     const size_t l3_bytes = sizeof(unsigned long long) * ((size_t)1 << s->l3_log);
@@ -944,6 +999,8 @@ extern "C" int mlmq_solver_create(const mlmq_graph *g, const mlmq_config *cfg_in
     if (!rc) rc = dev_alloc(&s->d_l3, l3_bytes, s->stream, "alloc(L3)");
     if (!rc) rc = dev_alloc(&s->d_l3bits, l3_bits_bytes(s->nids), s->stream, "alloc(L3 bits)");
     if (!rc) rc = dev_alloc(&s->d_ctl, sizeof(unsigned) * ctl::WORDS, s->stream, "alloc(ctl)");
+    if (!rc && s->owner_block)
+        rc = dev_alloc(&s->d_tails, owner_tails_bytes(owner_ctas), s->stream, "alloc(tails)");
     if (!rc) rc = pinned_ctl_alloc(&s->h_ctl);
     if (!rc) rc = fill_device(s->d_dist, g->n, INT_MAX, s->stream);
     if (!rc) rc = cuda_fail(cudaStreamSynchronize(s->stream), "solver init");
@@ -1021,7 +1078,9 @@ extern "C" int mlmq_solver_launch(mlmq_solver *s, int src, void *stream) {
     p.l3_log = s->l3_log;
     p.workers = s->workers;
     p.timeout_ns = (unsigned long long)s->cfg.timeout_ms * 1000000ull;
-    rc = cuda_fail(plain_launch(p, s->cfg.relax_unroll, s->grid, st), "persistent launch");
+    rc = s->owner_block
+             ? cuda_fail(owner_launch(p, s->owner_block, s->grid, s->d_tails, st), "owner launch")
+             : cuda_fail(plain_launch(p, s->cfg.relax_unroll, s->grid, st), "persistent launch");
     if (rc) {
         s->dirty = true;
         return rc;
@@ -1079,7 +1138,7 @@ extern "C" int mlmq_solver_stats(mlmq_solver *s, mlmq_solve_stats *st) {
     st->batches = c[ctl::ST_BATCHES];
     st->idle = c[ctl::ST_IDLE];
     st->grid = s->grid;
-    st->block = 32 * (s->workers + 1);
+    st->block = s->owner_block ? owner_threads() : 32 * (s->workers + 1);
     st->status = s->h_ctl[ctl::STATUS];
     return MLMQ_OK;
 }
@@ -1095,6 +1154,7 @@ extern "C" void mlmq_solver_destroy(mlmq_solver *s) {
     dev_free(s->d_l3, s->stream);
     dev_free(s->d_l3bits, s->stream);
     dev_free(s->d_ctl, s->stream);
+    dev_free(s->d_tails, s->stream);
     pinned_ctl_free(s->h_ctl);
     if (s->done) cudaEventDestroy(s->done);
     if (s->stream) cudaStreamDestroy(s->stream);
@@ -1205,7 +1265,7 @@ int dropin_run(int src) {
     if (src < 0 || src >= g_graph->n) return MLMQ_ERR_ARG;
     const char *qname = cfg.queue_type == MLMQ_L1V_L2DQ ? "L1V_L2DQ" : "L1SLF_L2DQ";
     std::printf("MLMQ_B200_CONFIG workers=%d blocks=%d delta=%d queue=%s\n",
-                32 * g_solver->workers, g_solver->grid, cfg.delta, qname);
+                g_solver->owner_block ? owner_threads() : 32 * g_solver->workers, g_solver->grid, cfg.delta, qname);
     const int warmups = env_int("BENCH_WARMUPS", 2, nullptr);
     const int repeats = env_int("BENCH_REPEATS", 3, nullptr);
     if (warmups < 0 || repeats < 1) return MLMQ_ERR_ARG;

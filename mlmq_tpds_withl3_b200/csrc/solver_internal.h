@@ -27,6 +27,10 @@ struct mlmq_graph {
     int4 *d_tiles = nullptr; // 2 per vertex and per piece: the vertex tiles (always owned)
     int pieces = 0;          // virtual vertices n .. n + pieces - 1 (split heavy vertices)
     int slots() const { return n + pieces; }
+    int max_degree = 0;
+    // Share of arcs (of a sample) that leave their tail's block of consecutive
+    // vertices, blocks as owner_block cuts them.
+    float away = 1.0f;
     // Per delta: light arcs (weight < delta) of each vertex, n ints.
     std::mutex split_mu;
     std::vector<std::pair<int, int *>> split_cache;
@@ -50,6 +54,8 @@ struct mlmq_solver {
     unsigned long long *d_l3 = nullptr;
     unsigned *d_l3bits = nullptr;  // one bit per vertex: the vertex has an L3 record
     unsigned *d_ctl = nullptr;
+    int owner_block = 0;        // vertices per CTA of the vertex-owner kernel; 0: not used
+    unsigned *d_tails = nullptr; // its inbox tails, a line per CTA
     unsigned *h_ctl = nullptr;  // pinned copy of the control block after each solve
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;

@@ -1,0 +1,629 @@
+// sssp_owner.cuh -- a single-source solve in which every vertex belongs to one
+// CTA, for graphs whose vertex numbering keeps neighbours together.
+//
+// CTA c owns the contiguous vertices [c * block, (c + 1) * block) and keeps
+// their distances in its shared memory for the whole solve.  A road-like graph
+// in row, Morton or breadth-first order has 1-5 % of its arcs between blocks of
+// some ten thousand vertices, so nearly every hop of the wavefront stays inside
+// one SM.  The CTA's worker warps relax in ticks: everything in the near list
+// is relaxed, what improves goes to the next tick's list, one barrier.  A tick
+// is a tile load, two rounds of shared-memory atomics and the barrier, about
+// 1.1 us (2100 cycles: list and distance 0.4k, tile 0.65k, minima and list
+// appends 0.7k, barrier and bookkeeping 0.3k), where a hop of the asynchronous
+// kernel (sssp_plain_body.cuh) takes about 2 us through two dependent global
+// round trips and its queues; and each CTA relaxes in order of distance, 1.2 to
+// 1.9 relaxations an arc against 2.2 to 9.  What bounds a solve is the number
+// of ticks along the wavefront's path times that latency, so every step inside
+// a tick that waits for the one before counts, not bytes.
+//
+// Measured on a B200 (default settings, source in the middle, one solve,
+// asynchronous kernel -> this one): grid 64^2 0.33 -> 0.14 ms, grid 512^2 2.00
+// -> 1.19 ms, grid 1200x777 6.1 -> 2.9 ms, grid 2048^2 10.5 -> 7.0 ms, kNN of
+// 100 000 points 1.04 -> 0.74 ms, of a million 3.6 -> 2.5 ms (64-byte tiles).
+//
+// Two arcs a lane: a vertex's tile is read by 2 (32-byte tiles) or 4 (64-byte)
+// lanes, 16 bytes each.  With a whole vertex per lane the four minima, list
+// appends and their branches ran one after another (0.25 ms on grid 64^2, 1.9
+// ms on grid 512^2).  24 worker warps: 16 leave two rounds where a list is long
+// (a million points 2.5 -> 2.7 ms).
+//
+// Arcs that leave the block become messages: the worker puts (vertex,
+// distance) in a shared-memory outbox, the CTA's sender warp appends it to the
+// owner's inbox ring in global memory (one returned atomic per destination,
+// one 64-bit compare-and-swap per record, as the L2 rings of mlmq_queue.cuh),
+// the owner's receiver warp moves it to a shared-memory inbox, and the
+// owner's workers apply it in their next tick.  Sender and receiver run beside
+// the ticks, so the round trips of a message never hold up local hops.
+//
+// Order inside a block: `near` holds the vertices to relax now, `far` those at
+// or beyond the threshold; when near runs empty the threshold moves to the
+// smallest far distance plus the bucket width.  A list entry carries half of
+// the distance that made it, so a vertex that has improved since is relaxed
+// once, at its newest entry.  A list without room sets the vertex's bit
+// instead, and the bits are taken up when the list has drained.
+//
+// The end: every message counts once in its inbox's tail when it is appended
+// and once in CREDIT when its owner has nothing left to do and has sent
+// everything that followed from it.  CTA 0's controller warp reads CREDIT and
+// then the tails; equality means that nothing is outstanding anywhere.
+#pragma once
+
+#include "mlmq_queue.cuh"
+
+namespace mlmq {
+
+constexpr int OWNER_WORKERS = 24;               // worker warps per CTA
+constexpr int OWNER_THREADS = 32 * (OWNER_WORKERS + 3);  // + sender, receiver, controller
+constexpr unsigned OWNER_T = 32u * OWNER_WORKERS;
+constexpr unsigned OWNER_NEAR = 2048;           // list entries
+constexpr unsigned OWNER_FAR = 3072;
+constexpr unsigned OWNER_OUT = 512;             // outbox and inbox records
+constexpr unsigned OWNER_IN = 512;
+// Ticks a bucket above (below) which the next one is half (twice) as wide.
+constexpr unsigned OWNER_LONG = 48, OWNER_SHORT = 20;
+// The first bucket is this fraction of the configured width.
+constexpr unsigned OWNER_START = 16;
+// Most vertices of a block: 16-bit ids, and distances, two bits a vertex and the
+// lists within 227 KB.
+constexpr int OWNER_MAX_BLOCK = 43008;
+
+struct OwnerParams {
+    unsigned block, block_inv;  // vertices per CTA (a multiple of 32), (2^32 - 1) / block
+    int inbox_log;              // log2 slots of one inbox ring
+    unsigned *tails;            // [CTAs] one 128-byte line each
+};
+
+// Shared memory: distances, near bits, far bits, near lists, far lists.
+__host__ __device__ constexpr size_t owner_smem_bytes(unsigned block) {
+    return (size_t)block * 4 + (size_t)(block / 32) * 8 + 2 * 4 * (size_t)OWNER_NEAR +
+           2 * 4 * (size_t)OWNER_FAR + 8 * (size_t)(OWNER_OUT + OWNER_IN);
+}
+
+// What a tick begins with, read whole: tick t uses entry t mod 3, pushes of the
+// tick before count into `n`, worker 0's view of the inbox and the exit flag
+// is written then too.
+struct alignas(16) OwnerTick {
+    unsigned n, in_tail, exit, pad;
+};
+
+struct OwnerShared {
+    OwnerTick tick[3];
+    unsigned far_n[2];
+    unsigned in_tail, in_head;    // inbox: written by the receiver / by worker 0
+    unsigned out_tail, out_sent;  // outbox: written by the workers / by the sender
+    unsigned exit;        // set by the receiver: leave
+    unsigned least[2];    // smallest far distance, by tick parity
+    unsigned near_over;   // near bits without a list entry exist
+    unsigned range;
+    unsigned long long pushed, relaxed, sent;
+};
+
+__device__ __forceinline__ void owner_bar() {
+    asm volatile("bar.sync 1, %0;" ::"n"(OWNER_T) : "memory");
+}
+__device__ __forceinline__ uint4 ld_shared4(const void *p) {
+    uint4 v;
+    asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned ld_shared(const unsigned *p) {
+    return *reinterpret_cast<const volatile unsigned *>(p);
+}
+
+struct Owner {
+    const PlainParams &p;
+    const OwnerParams &o;
+    OwnerShared &sh;
+    unsigned lo, cnt;     // first vertex and vertices of the block
+    int *dist;
+    unsigned *near_bits, *far_bits;
+    unsigned *near_list, *far_list;  // two lists each
+    unsigned long long *out, *in;
+    unsigned thr;         // near holds distances below it
+    unsigned next_slot;   // near_n index and list half that pushes go to
+    unsigned next_half, far_half;
+    unsigned pushed, relaxed, sent;
+    bool range;
+};
+
+__device__ __forceinline__ unsigned shared_addr(const void *p) {
+    return (unsigned)__cvta_generic_to_shared(p);
+}
+// A predicated shared-memory minimum: straight-line code, so that a lane's two
+// are in flight together.  Returns INT_MIN when off.
+__device__ __forceinline__ int shared_min(bool on, unsigned addr, int v) {
+    int r = INT_MIN;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t"
+                 "@q atom.shared.min.s32 %0, [%1], %2;\n\t}"
+                 : "+r"(r) : "r"(addr), "r"(v), "r"((unsigned)on) : "memory");
+    return r;
+}
+
+// A list entry: the local id and the low half of the distance that put it
+// there.  A vertex that has improved since has a newer entry; the old one is
+// told by its half (an equal half of another distance costs a relaxation
+// twice, never a result).
+__device__ __forceinline__ unsigned owner_entry(unsigned l, unsigned d) { return (d << 16) | l; }
+__device__ __forceinline__ bool owner_live(unsigned entry, unsigned d) {
+    return ((entry >> 16) ^ d) << 16 == 0u;
+}
+
+// Up to N records per lane for the lists, by a whole warp: vertex l[k] to the
+// near list of the next tick (near[k]) or to far (far[k]).  One shared-memory
+// add gives the warp's places in both lists.
+template <int N>
+__device__ __forceinline__ void owner_append(Owner &w, const bool (&near)[N], const bool (&far)[N],
+                                             const unsigned (&l)[N], const unsigned (&d)[N]) {
+    const unsigned lane = threadIdx.x & 31u;
+    unsigned nm[N], fm[N], nn = 0, fn = 0;
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        nm[k] = __ballot_sync(FULL, near[k]);
+        fm[k] = __ballot_sync(FULL, far[k]);
+        nn += (unsigned)__popc(nm[k]);
+        fn += (unsigned)__popc(fm[k]);
+    }
+    if ((nn | fn) == 0u) return;
+    unsigned at = 0;
+    if (lane < 2u)
+        at = atomicAdd(lane ? w.sh.far_n + w.far_half : &w.sh.tick[w.next_slot].n, lane ? fn : nn);
+    unsigned an = __shfl_sync(FULL, at, 0), af = __shfl_sync(FULL, at, 1);
+    const bool full = an + nn > OWNER_NEAR || af + fn > OWNER_FAR;
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        const unsigned i = near[k] ? an + (unsigned)__popc(nm[k] & lanemask_lt())
+                                   : af + (unsigned)__popc(fm[k] & lanemask_lt());
+        if (near[k] || far[k]) {
+            if (!full || i < (near[k] ? OWNER_NEAR : OWNER_FAR)) {
+                (near[k] ? w.near_list + w.next_half * OWNER_NEAR
+                         : w.far_list + w.far_half * OWNER_FAR)[i] = owner_entry(l[k], d[k]);
+            } else {
+                // No room: the vertex's bit stands for it until the list has
+                // drained.
+                atomicOr((near[k] ? w.near_bits : w.far_bits) + (l[k] >> 5), 1u << (l[k] & 31u));
+            }
+        }
+        an += (unsigned)__popc(nm[k]);
+        af += (unsigned)__popc(fm[k]);
+    }
+}
+
+// Up to N candidates per lane for vertices of this block (local id l[k],
+// distance d[k] below INT_MAX, when on[k]).
+template <int N>
+__device__ __forceinline__ void owner_update(Owner &w, const bool (&on)[N], const unsigned (&l)[N],
+                                             const unsigned (&d)[N]) {
+    const unsigned dist = shared_addr(w.dist);
+    int before[N];
+    bool near[N], far[N];
+#pragma unroll
+    for (int k = 0; k < N; k++) before[k] = shared_min(on[k], dist + 4u * l[k], (int)d[k]);
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        const bool win = (int)d[k] < before[k];
+        w.pushed += win;
+        near[k] = win && d[k] < w.thr;
+        far[k] = win && d[k] >= w.thr;
+    }
+    owner_append<N>(w, near, far, l, d);
+}
+
+// A message for the owner of `v`.  Waits (the sender warp keeps draining) while
+// the outbox is full.
+__device__ __forceinline__ void owner_send(Owner &w, unsigned v, unsigned d,
+                                           unsigned long long deadline) {
+    const unsigned i = atomicAdd(&w.sh.out_tail, 1u);
+    w.sent++;
+    unsigned polls = 0;
+    while (i - ld_shared(&w.sh.out_sent) >= OWNER_OUT) {
+        if (ld_shared(&w.sh.exit)) return;
+        if ((++polls & 255u) == 0u && globaltimer() > deadline) return;
+    }
+    *reinterpret_cast<volatile unsigned long long *>(w.out + (i & (OWNER_OUT - 1u))) =
+        ((unsigned long long)d << 32) | v;
+}
+
+// Relaxes two arcs per lane from distance d (a whole warp).
+__device__ __forceinline__ void owner_arcs(Owner &w, const bool (&ok)[2], const unsigned (&u)[2],
+                                           const unsigned (&nd)[2], unsigned long long deadline) {
+    bool here[2], away = false, big = false;
+    unsigned l[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        l[k] = u[k] - w.lo;
+        const bool fits = nd[k] < (unsigned)INT_MAX;
+        here[k] = ok[k] && l[k] < w.cnt && fits;
+        away |= ok[k] && l[k] >= w.cnt;
+        big |= ok[k] && !fits;
+        w.relaxed += ok[k];
+    }
+    owner_update<2>(w, here, l, nd);
+    if (__any_sync(FULL, away || big)) {
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            if (!ok[k]) continue;
+            if (l[k] >= w.cnt) owner_send(w, u[k], min(nd[k], (unsigned)INT_MAX), deadline);
+            else if (nd[k] >= (unsigned)INT_MAX && w.dist[l[k]] == INT_MAX)
+                w.range = true;  // a finite distance would not fit
+        }
+        __syncwarp();
+    }
+}
+
+// Relaxes the vertices of near entries [i0, i0 + 32 / LPV) of `list` that are
+// below n, LPV lanes each, two arcs per lane.
+template <class Arcs, int LPV>
+__device__ __forceinline__ void owner_relax(Owner &w, const unsigned *list, unsigned i0,
+                                            unsigned n, unsigned long long deadline) {
+    const PlainParams &p = w.p;
+    const unsigned lane = threadIdx.x & 31u, sub = lane % LPV;
+    const unsigned i = i0 + lane / LPV;
+    const unsigned entry = i < n ? list[i] : 0u;
+    const unsigned l = entry & 0xffffu;
+    const unsigned v = w.lo + l;
+    int beg = 0, deg = 0;
+    int4 t = make_int4(-1, 0, -1, 0);
+    if (p.tiles && i < n) t = __ldg(p.tiles + (size_t)LPV * v + sub);
+    const unsigned d = (unsigned)*reinterpret_cast<volatile int *>(w.dist + l);
+    const bool valid = i < n && owner_live(entry, d);
+    if (p.tiles) {
+        if (!valid) t = make_int4(-1, 0, -1, 0);
+        const bool csr = sub == 0 && t.x == TILE_CSR;
+        if (csr) {
+            beg = t.y;
+            deg = t.z;
+        }
+        const unsigned cm = __ballot_sync(FULL, csr);
+        const unsigned u[2] = {(unsigned)t.x, (unsigned)t.z};
+        const unsigned nd[2] = {d + (unsigned)t.y, d + (unsigned)t.w};
+        const bool ok[2] = {t.x >= 0, !csr && t.z >= 0};
+        owner_arcs(w, ok, u, nd, deadline);
+        if (cm == 0u) return;
+    } else {
+        if (valid && sub == 0) {
+            beg = __ldg(p.row + v);
+            deg = __ldg(p.row + v + 1) - beg;
+        }
+    }
+    // CSR ranges: the vertex's lanes take two arcs each in turn.
+    beg = __shfl_sync(FULL, beg, (int)(lane - sub));
+    deg = __shfl_sync(FULL, deg, (int)(lane - sub));
+    for (int g = 0; __any_sync(FULL, g < deg); g += 2 * LPV) {
+        const int e = g + 2 * (int)sub;
+        const bool ok[2] = {e < deg, e + 1 < deg};
+        const int2 a = ok[0] ? Arcs::load(p, beg + e) : make_int2(0, 0);
+        const int2 b = ok[1] ? Arcs::load(p, beg + e + 1) : make_int2(0, 0);
+        const unsigned u[2] = {(unsigned)a.x, (unsigned)b.x};
+        const unsigned nd[2] = {d + (unsigned)a.y, d + (unsigned)b.y};
+        owner_arcs(w, ok, u, nd, deadline);
+    }
+}
+
+// The smallest distance among the far vertices, 0xffffffff if there is none: by
+// every lane's share of the `n` list entries, and of the bits if `over`.
+__device__ __forceinline__ unsigned owner_least(const Owner &w, unsigned tid, bool over, unsigned n) {
+    const unsigned words = (w.cnt + 31u) >> 5;
+    const unsigned *list = w.far_list + w.far_half * OWNER_FAR;
+    unsigned least = 0xffffffffu;
+    for (unsigned i = tid; i < n; i += OWNER_T) {
+        const unsigned entry = list[i], d = (unsigned)w.dist[entry & 0xffffu];
+        if (d >= w.thr && owner_live(entry, d)) least = min(least, d);
+    }
+    if (over)
+        for (unsigned i = tid; i < words; i += OWNER_T)
+            for (unsigned b = w.far_bits[i]; b; b &= b - 1u) {
+                const unsigned d = (unsigned)w.dist[32u * i + (unsigned)__ffs(b) - 1u];
+                if (d >= w.thr) least = min(least, d);
+            }
+    return __reduce_min_sync(FULL, least);
+}
+
+// Raises the threshold to `thr` and moves the far vertices below it to the near
+// list of the next tick, the others to the other far list.  One whose distance
+// is below the old threshold was relaxed from near in the meantime.
+__device__ __forceinline__ void owner_raise(Owner &w, unsigned tid, bool over, unsigned n,
+                                            unsigned thr) {
+    const unsigned old = w.thr, words = (w.cnt + 31u) >> 5;
+    const unsigned *list = w.far_list + w.far_half * OWNER_FAR;
+    w.far_half ^= 1u;
+    w.thr = thr;
+    for (unsigned i0 = tid & ~31u; i0 < n; i0 += OWNER_T) {
+        const unsigned i = i0 + (tid & 31u);
+        const unsigned entry = i < n ? list[i] : 0u;
+        const unsigned l[1] = {entry & 0xffffu};
+        const unsigned d[1] = {(unsigned)w.dist[l[0]]};
+        const bool live = i < n && owner_live(entry, d[0]);
+        const bool near[1] = {live && d[0] >= old && d[0] < thr}, far[1] = {live && d[0] >= thr};
+        owner_append<1>(w, near, far, l, d);
+    }
+    if (over)
+        for (unsigned i0 = tid & ~31u; i0 < words; i0 += OWNER_T) {
+            const unsigned i = i0 + (tid & 31u);
+            unsigned b = 0;
+            // The bits are taken before any is set again for want of room.
+            if (i < words) b = atomicExch(w.far_bits + i, 0u);
+            while (__any_sync(FULL, b != 0u)) {
+                const unsigned l[1] = {b ? 32u * i + (unsigned)__ffs(b) - 1u : 0u};
+                const unsigned d[1] = {(unsigned)w.dist[l[0]]};
+                const bool near[1] = {b != 0u && d[0] >= old && d[0] < thr},
+                           far[1] = {b != 0u && d[0] >= thr};
+                owner_append<1>(w, near, far, l, d);
+                b &= b - 1u;
+            }
+        }
+}
+
+template <class Arcs, int LPV>
+__device__ __forceinline__ void owner_work(Owner &w, unsigned long long deadline) {
+    OwnerShared &sh = w.sh;
+    const unsigned tid = threadIdx.x;
+    // The last warp has entries to relax least often: its lane 0 keeps the books.
+    const bool clerk = tid == OWNER_T - 32u;
+    unsigned done_in = 0;      // messages applied (uniform)
+    unsigned returned = 0;     // of which credited (the clerk)
+    unsigned ticks = 0, width = w.thr;
+    const unsigned width_max = (unsigned)min(0x3fffffffull, (unsigned long long)w.p.delta * (unsigned)w.p.bm);
+    unsigned slot = 0;  // t mod 3
+    uint4 head = ld_shared4(&sh.tick[0]);
+    for (unsigned t = 0;; t++) {
+        // `head` was written before the last barrier.
+        const unsigned n = min(head.x, OWNER_NEAR), tail = head.y;
+        if (head.z) break;
+        w.next_slot = slot == 2u ? 0u : slot + 1u;
+        w.next_half = (t + 1u) & 1u;
+        if (clerk) {
+            if (head.x > OWNER_NEAR) sh.near_over = 1u;
+            *reinterpret_cast<volatile unsigned *>(&sh.in_head) = done_in;
+            sh.tick[w.next_slot].in_tail = ld_shared(&sh.in_tail);
+            sh.tick[w.next_slot].exit = ld_shared(&sh.exit);
+            sh.least[(t + 1u) & 1u] = 0xffffffffu;
+            sh.tick[w.next_slot == 2u ? 0u : w.next_slot + 1u].n = 0u;
+        }
+        // Messages that have arrived.
+        for (unsigned i0 = done_in + (tid & ~31u); (int)(tail - i0) > 0; i0 += OWNER_T) {
+            const unsigned i = i0 + (tid & 31u);
+            const bool mine = (int)(tail - i) > 0;
+            const unsigned long long r = mine ? w.in[i & (OWNER_IN - 1u)] : 0ull;
+            const unsigned l[1] = {(unsigned)r - w.lo}, d[1] = {(unsigned)(r >> 32)};
+            const bool on[1] = {mine && d[0] < (unsigned)INT_MAX};
+            if (mine && !on[0] && w.dist[l[0]] == INT_MAX) w.range = true;
+            owner_update<1>(w, on, l, d);
+        }
+        done_in = tail;
+        const unsigned *list = w.near_list + (t & 1u) * OWNER_NEAR;
+        for (unsigned i0 = (tid >> 5) * (32u / LPV); i0 < n; i0 += OWNER_T / LPV)
+            owner_relax<Arcs, LPV>(w, list, i0, n, deadline);
+        ticks += n != 0u;
+        owner_bar();
+        slot = w.next_slot;
+        head = ld_shared4(&sh.tick[slot]);
+        if (head.x != 0u) continue;
+        // Near is empty.
+        const unsigned far = ld_shared(sh.far_n + w.far_half);
+        const bool over = ld_shared(&sh.near_over) != 0u;
+        owner_bar();
+        if (over) {
+            // The vertices that had no room in the list.
+            if (clerk) sh.near_over = 0u;
+            const unsigned words = (w.cnt + 31u) >> 5;
+            for (unsigned i0 = tid & ~31u; i0 < words; i0 += OWNER_T) {
+                const unsigned i = i0 + (tid & 31u);
+                unsigned b = i < words ? atomicExch(w.near_bits + i, 0u) : 0u;
+                while (__any_sync(FULL, b != 0u)) {
+                    const unsigned l[1] = {b ? 32u * i + (unsigned)__ffs(b) - 1u : 0u};
+                    const unsigned d[1] = {(unsigned)w.dist[l[0]]};
+                    const bool near[1] = {b != 0u}, none[1] = {false};
+                    owner_append<1>(w, near, none, l, d);
+                    b &= b - 1u;
+                }
+            }
+            owner_bar();
+        } else if (far != 0u) {
+            // The next bucket begins at the smallest far distance.
+            if (clerk) sh.far_n[w.far_half ^ 1u] = 0u;
+            const unsigned listed = min(far, OWNER_FAR);
+            const unsigned mine = owner_least(w, tid, far > OWNER_FAR, listed);
+            if ((tid & 31u) == 0u && mine != 0xffffffffu) atomicMin(&sh.least[t & 1u], mine);
+            owner_bar();
+            const unsigned least = ld_shared(&sh.least[t & 1u]);
+            // A bucket switch costs about a tick.  Many ticks a bucket: a finer
+            // order is nearly free; few: the switches are what takes time.
+            if (ticks > OWNER_LONG && width > 1u) width >>= 1;
+            else if (ticks < OWNER_SHORT && width < width_max) width = min(2u * width, width_max);
+            ticks = 0;
+            owner_raise(w, tid, far > OWNER_FAR, listed,
+                        least == 0xffffffffu ? w.thr : max(least + 1u, min(least + width, 0x7fffffffu)));
+            owner_bar();
+        } else if (clerk) {
+            // Nothing to do: what the applied messages led to has been sent
+            // once the outbox is empty, so their credit may go back.
+            if (done_in != returned && ld_shared(&sh.out_sent) == ld_shared(&sh.out_tail)) {
+                __threadfence();
+                atomicAdd(w.p.ctlw + ctl::CREDIT, done_in - returned);
+                returned = done_in;
+            }
+        }
+        head.x = ld_shared(&sh.tick[slot].n);
+    }
+}
+
+// The sender warp: outbox records to their owners' inbox rings.
+__device__ __forceinline__ void owner_sender(const PlainParams &p, const OwnerParams &o,
+                                             OwnerShared &sh, unsigned long long *out,
+                                             unsigned long long deadline) {
+    const unsigned lane = threadIdx.x & 31u;
+    unsigned at = 0;
+    for (;;) {
+        volatile unsigned long long *slot = out + ((at + lane) & (OWNER_OUT - 1u));
+        const unsigned long long r = *slot;
+        const unsigned okm = __ballot_sync(FULL, r != SENT);
+        const unsigned k = okm == FULL ? 32u : (unsigned)__ffs(~okm) - 1u;
+        if (k == 0u) {
+            if (ld_shared(&sh.exit)) return;
+            __nanosleep(32);
+            continue;
+        }
+        const bool mine = lane < k;
+        const unsigned v = (unsigned)r, d = (unsigned)(r >> 32);
+        unsigned c = 0xffffffffu;
+        if (mine) {
+            *slot = SENT;
+            c = __umulhi(v, o.block_inv);  // at most one too small
+            if (v - c * o.block >= o.block) c++;
+        }
+        const unsigned grp = __match_any_sync(FULL, c);
+        const unsigned leader = (unsigned)__ffs(grp) - 1u;
+        unsigned pos = 0;
+        if (mine && lane == leader) pos = atomicAdd(o.tails + 32u * c, (unsigned)__popc(grp));
+        pos = __shfl_sync(FULL, pos, leader) + __popc(grp & lanemask_lt());
+        if (mine) {
+            unsigned long long *to =
+                p.l2 + ((size_t)c << o.inbox_log) + (pos & ((1u << o.inbox_log) - 1u));
+            const unsigned long long rec = rec_pack(v, d, pos >> o.inbox_log);
+            if (atomicCAS(to, SENT, rec) != SENT) install_slow(p, to, rec, deadline);
+        }
+        __syncwarp();
+        at += k;
+        if (lane == 0) {
+            __threadfence_block();
+            *reinterpret_cast<volatile unsigned *>(&sh.out_sent) = at;
+        }
+    }
+}
+
+// The receiver warp: this CTA's inbox ring to the shared-memory inbox; it also
+// brings the end of the solve to the CTA.
+__device__ __forceinline__ void owner_receiver(const PlainParams &p, const OwnerParams &o,
+                                               OwnerShared &sh, unsigned long long *in) {
+    const unsigned lane = threadIdx.x & 31u;
+    unsigned long long *ring = p.l2 + ((size_t)blockIdx.x << o.inbox_log);
+    const unsigned mask = (1u << o.inbox_log) - 1u;
+    unsigned at = 0;
+    for (;;) {
+        const unsigned ex = lane == 0u ? ld_relaxed(p.ctlw + ctl::EXIT) : 0u;
+        const unsigned s = at + lane;
+        unsigned long long r = SENT;
+        const unsigned room = OWNER_IN - (at - ld_shared(&sh.in_head));
+        if (lane < room) r = ld_relaxed64(ring + (s & mask));
+        const bool ok = r != SENT && rec_lap(r) == ((s >> o.inbox_log) & 3u);
+        const unsigned okm = __ballot_sync(FULL, ok);
+        const unsigned k = okm == FULL ? 32u : (unsigned)__ffs(~okm) - 1u;
+        if (lane < k) {
+            st_relaxed64(ring + (s & mask), SENT);
+            in[s & (OWNER_IN - 1u)] = ((unsigned long long)rec_d(r) << 32) | rec_v(r);
+        }
+        __syncwarp();
+        if (k) {
+            at += k;
+            if (lane == 0) {
+                __threadfence_block();
+                *reinterpret_cast<volatile unsigned *>(&sh.in_tail) = at;
+            }
+        }
+        if (__shfl_sync(FULL, ex, 0)) {
+            if (lane == 0) *reinterpret_cast<volatile unsigned *>(&sh.exit) = 1u;
+            return;
+        }
+    }
+}
+
+// CTA 0's controller warp: the end of the solve and the time limit.
+__device__ __forceinline__ void owner_controller(const PlainParams &p, const OwnerParams &o,
+                                                 unsigned long long deadline) {
+    const unsigned lane = threadIdx.x & 31u;
+    for (;;) {
+        // CREDIT before the tails: a credit is returned only after the sends
+        // it covers, so any credit seen here comes with their tails and the
+        // difference can only overstate what is outstanding.
+        const unsigned credit = ld_acquire(p.ctlw + ctl::CREDIT);
+        __syncwarp();
+        unsigned sum = 0;
+        for (unsigned c = lane; c < gridDim.x; c += 32) sum += ld_relaxed(o.tails + 32u * c);
+        sum = __reduce_add_sync(FULL, sum);
+        if (sum == __shfl_sync(FULL, credit, 0)) {
+            if (lane == 0) {
+                atomicOr(p.ctlw + ctl::STATUS, ST_DONE);
+                st_release(p.ctlw + ctl::EXIT, 1u);
+            }
+            return;
+        }
+        if (globaltimer() > deadline) {
+            if (lane == 0) raise_status(p, ST_TIMEOUT);
+            return;
+        }
+        if (__shfl_sync(FULL, ld_relaxed(p.ctlw + ctl::EXIT), 0)) return;
+    }
+}
+
+template <class Arcs, int LPV>
+__device__ __forceinline__ void owner_solve(const PlainParams &p, const OwnerParams &o) {
+    extern __shared__ unsigned long long owner_smem[];
+    __shared__ OwnerShared sh;
+    const unsigned tid = threadIdx.x, warp = tid >> 5;
+    const unsigned long long deadline = globaltimer() + p.timeout_ns;
+    Owner w{p, o, sh};
+    w.lo = blockIdx.x * o.block;
+    w.cnt = min(o.block, (unsigned)p.n - min(w.lo, (unsigned)p.n));
+    w.out = owner_smem;
+    w.in = w.out + OWNER_OUT;
+    w.dist = reinterpret_cast<int *>(w.in + OWNER_IN);
+    w.near_bits = reinterpret_cast<unsigned *>(w.dist + o.block);
+    w.far_bits = w.near_bits + o.block / 32u;
+    w.near_list = w.far_bits + o.block / 32u;
+    w.far_list = w.near_list + 2 * OWNER_NEAR;
+    w.next_slot = w.next_half = w.far_half = 0u;
+    w.pushed = w.relaxed = w.sent = 0u;
+    w.range = false;
+    // The first bucket is a fraction of the configured width, which is the
+    // most that later ones may grow to.
+    w.thr = max(1u, p.delta / OWNER_START);
+    for (unsigned i = tid; i < o.block; i += OWNER_THREADS) w.dist[i] = INT_MAX;
+    for (unsigned i = tid; i < o.block / 32u; i += OWNER_THREADS) w.near_bits[i] = w.far_bits[i] = 0u;
+    for (unsigned i = tid; i < OWNER_OUT; i += OWNER_THREADS) w.out[i] = SENT;
+    if (tid == 0) {
+        for (int i = 0; i < 3; i++) sh.tick[i] = OwnerTick{0u, 0u, 0u, 0u};
+        sh.least[0] = sh.least[1] = 0xffffffffu;
+        sh.far_n[0] = sh.far_n[1] = 0u;
+        sh.in_tail = sh.in_head = sh.out_tail = sh.out_sent = 0u;
+        sh.exit = sh.near_over = sh.range = 0u;
+        sh.pushed = sh.relaxed = sh.sent = 0ull;
+    }
+    if (blockIdx.x == 0) {
+        for (int i = (int)tid; i < ctl::WORDS; i += OWNER_THREADS)
+            if (i != ctl::BAR_COUNT && i != ctl::BAR_GEN) p.ctlw[i] = 0u;
+        // The source is the first message, to its owner's inbox.
+        const unsigned c = (unsigned)p.src / o.block;
+        for (unsigned i = tid; i < gridDim.x; i += OWNER_THREADS) o.tails[32u * i] = i == c;
+        if (tid == 0) p.l2[(size_t)c << o.inbox_log] = rec_pack((unsigned)p.src, 0u, 0u);
+    }
+    if (!grid_barrier(p.ctlw, gridDim.x, deadline)) return;
+
+    if (warp < OWNER_WORKERS) owner_work<Arcs, LPV>(w, deadline);
+    else if (warp == OWNER_WORKERS) owner_sender(p, o, sh, w.out, deadline);
+    else if (warp == OWNER_WORKERS + 1) owner_receiver(p, o, sh, w.in);
+    else if (blockIdx.x == 0) owner_controller(p, o, deadline);
+
+    __syncthreads();
+    for (unsigned i = tid; i < w.cnt; i += OWNER_THREADS) p.dist[w.lo + i] = w.dist[i];
+    const unsigned pushed = __reduce_add_sync(FULL, w.pushed);
+    const unsigned relaxed = __reduce_add_sync(FULL, w.relaxed);
+    const unsigned sent = __reduce_add_sync(FULL, w.sent);
+    if (w.range) sh.range = 1u;
+    if ((tid & 31u) == 0) {
+        atomicAdd(&sh.pushed, (unsigned long long)pushed);
+        atomicAdd(&sh.relaxed, (unsigned long long)relaxed);
+        atomicAdd(&sh.sent, (unsigned long long)sent);
+    }
+    __syncthreads();
+    if (tid == 0) {
+        unsigned long long *st = reinterpret_cast<unsigned long long *>(p.ctlw + ctl::STATS);
+        atomicAdd(st + ctl::ST_PUSHED, sh.pushed + sh.sent);
+        atomicAdd(st + ctl::ST_RELAXED, sh.relaxed);
+        atomicAdd(st + ctl::ST_IMPROVED, sh.pushed);
+        if (sh.range) atomicOr(p.ctlw + ctl::STATUS, ST_RANGE);
+    }
+}
+
+}  // namespace mlmq

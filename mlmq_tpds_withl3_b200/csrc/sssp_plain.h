@@ -31,4 +31,14 @@ cudaError_t plain_max_blocks_per_sm(int workers, int unroll, int *blocks);
 // Cooperative launch of `grid` CTAs on `stream`.
 cudaError_t plain_launch(const PlainParams &p, int unroll, int grid, cudaStream_t stream);
 
+// The vertex-owner kernel (sssp_owner.cuh).  owner_block: vertices per CTA (a
+// multiple of 32) and CTAs for n vertices, 0 if they do not fit; owner_prepare
+// sets the kernels' shared-memory limit, before the first launch.
+int owner_threads();
+int owner_block(int n, int sms, int *ctas);
+size_t owner_tails_bytes(int ctas);
+cudaError_t owner_prepare();
+cudaError_t owner_launch(const PlainParams &p, int block, int ctas, unsigned *tails,
+                         cudaStream_t stream);
+
 }  // namespace mlmq

@@ -1,0 +1,92 @@
+"""The vertex-owner kernel (blocks of consecutive vertices, distances in shared
+memory, messages between blocks) against the oracle, at the sizes where it can
+go wrong; every comparison is exact int32 equality."""
+import numpy as np
+import pytest
+
+import oracle_lib
+from mlmq_tpds_withl3_b200 import DeviceGraph, HostGraph, MlmqError, Solver
+from mlmq_tpds_withl3_b200._lib import MLMQ_ERR_RANGE
+
+pytestmark = pytest.mark.gpu
+THREADS = 864  # of a vertex-owner CTA; the asynchronous kernel's are 32 * (workers + 1)
+
+
+def _csr(n, src, dst, w, name):
+    order = np.lexsort((dst, src))
+    src, dst, w = src[order], dst[order], w[order]
+    row = np.zeros(n + 1, np.int64)
+    row[1:] = np.cumsum(np.bincount(src, minlength=n))
+    return HostGraph.from_csr(row, dst, w, name)
+
+
+def _band(n, deg, reach, wmax, seed):
+    """Each vertex to `deg` random ones at most `reach` ids away."""
+    rng = np.random.default_rng(seed)
+    src = np.repeat(np.arange(n), deg)
+    dst = np.clip(src + rng.integers(-reach, reach + 1, n * deg), 0, n - 1)
+    return _csr(n, src, dst, rng.integers(0, wmax + 1, n * deg), f"band{n}")
+
+
+def _owned(solver):
+    return solver.stats()["block"] == THREADS
+
+
+@pytest.mark.parametrize("wide,high", [(2, 1), (31, 1), (32, 1), (33, 1), (128, 128), (16385, 1),
+                                       (127, 259), (181, 1021), (1021, 181)])
+def test_grids_at_block_edges(wide, high):
+    g = HostGraph.grid(wide, high, drop_p=0.0 if high == 1 else 0.1, seed=wide)
+    s = Solver(DeviceGraph.upload(g))
+    for src in (0, g.n // 2, g.n - 1):
+        ref, work = oracle_lib.sssp_i32(g, src)
+        assert np.array_equal(s.solve(src).dist(), ref), src
+        assert _owned(s) and s.stats()["relaxed"] >= work
+
+
+# Degrees beyond a tile, one weight for all (many equal candidates) and wide
+# ones, and wavefronts longer than the lists, the outbox and the inbox.
+@pytest.mark.parametrize("n,deg,reach,wmax", [(3000, 3, 40, 9), (16384, 24, 8000, 1),
+                                              (16384, 24, 8000, 10**6), (70001, 9, 1500, 10**5),
+                                              (70001, 30, 1900, 0), (40000, 6, 900, 5)])
+@pytest.mark.parametrize("cfg", [{}, {"vertex_tiles": 0}, {"vertex_tiles": 2, "delta": 1 << 30},
+                                 {"delta": 3}])
+def test_bands(n, deg, reach, wmax, cfg):
+    g = _band(n, deg, reach, wmax, n + deg)
+    s = Solver(DeviceGraph.upload(g), cfg)
+    for src in (0, n // 2):
+        ref, _ = oracle_lib.sssp_i32(g, src)
+        assert np.array_equal(s.solve(src).dist(), ref), src
+        assert _owned(s)
+
+
+def test_solves_share_the_workspace_with_other_graphs_and_orders():
+    """A local order and a shuffled one (asynchronous kernel) of the same
+    graph, solved in turn, give the same distances."""
+    g = HostGraph.grid(300, 250, seed=3)
+    perm = np.random.default_rng(1).permutation(g.n)
+    src = np.repeat(np.arange(g.n), np.diff(g.row))
+    mixed = _csr(g.n, perm[src], perm[g.col], g.w, "shuffled")
+    a, b = Solver(DeviceGraph.upload(g)), Solver(DeviceGraph.upload(mixed))
+    ref, _ = oracle_lib.sssp_i32(g, 77)
+    for _ in range(3):
+        assert np.array_equal(a.solve(77).dist(), ref)
+        assert np.array_equal(b.solve(int(perm[77])).dist()[perm], ref)
+    assert _owned(a) and not _owned(b)
+    split = Solver(a.graph, {"light_heavy": 1, "bucket_sync": 1})
+    assert np.array_equal(split.solve(77).dist(), ref) and not _owned(split)
+
+
+@pytest.mark.parametrize("first,second", [(100, 200), (16383, 32767)])
+def test_sums_beyond_the_range_are_reported(first, second):
+    """A path with two arcs of 2^30: inside a block, and between blocks."""
+    n = 40000
+    w = np.ones(n - 1, np.int64)
+    w[[first, second]] = 1 << 30
+    g = _csr(n, np.arange(n - 1), np.arange(1, n), w, "path")
+    s = Solver(DeviceGraph.upload(g))
+    with pytest.raises(MlmqError) as ei:
+        s.solve(0)
+    assert ei.value.code == MLMQ_ERR_RANGE
+    del ei
+    assert np.array_equal(s.solve(second + 1).dist(), oracle_lib.sssp_i32(g, second + 1)[0])
+    assert _owned(s)
