@@ -10,23 +10,35 @@
 // A FIFO search discovers the vertices of one level in the order of their
 // first discovering arc: (queue position of the parent, index of the arc in
 // the parent's row).  The device search is level-synchronous and reproduces
-// that order exactly:
-//   1. every arc out of the current level's vertices (queue positions
-//      [lo, hi), which ARE their new ids) proposes the key
-//      position << 32 | arc index to its undiscovered target with a 64-bit
-//      atomicMin; the first proposal to a target also appends it to the
-//      level's candidate list;
-//   2. the candidates are sorted by key (CUB radix sort): that is their
-//      discovery order, so candidate i gets new id hi + i;
-//   3. the next level is [hi, hi + count).
+// that order exactly.  Every arc out of the current level's vertices (queue
+// positions [lo, hi), which ARE their new ids) proposes the key
+// position << 32 | arc index to its target with a 64-bit atomicMin; a vertex
+// found at an earlier level keeps its smaller key.
+//   * Narrow levels run one after another in one CTA (up to NARROW_CAP
+//     vertices) or one cluster of eight (up to MIDDLE_CAP), none with a vertex
+//     of more than NARROW_DEGREE arcs, a vertex per thread: after a barrier the
+//     arc whose key stands discovers its target, and a scan in queue order
+//     gives the new ids -- no sort, no launches, no host.  A level is a chain
+//     of three global round trips (destinations; keys, with the targets' row
+//     offsets beside them; the keys again), a scan and the barriers, where a
+//     level of launches below costs about 35 us of launches, a sort of a
+//     thousand keys and a host round trip, and a road-like graph has thousands
+//     of levels: 1024 x 1024 grid 65.6 -> 7.9 ms, about 5 us a level.  One CTA
+//     is bound by its SM's rate of scattered atomics from about a thousand
+//     vertices a level on (all levels in one CTA: 1024 x 1024 16 ms, 4000 x 4000
+//     240 ms against 49 with the cluster), the cluster by its three barriers.
+//   * Wide levels use the whole device: the first proposal to a target also
+//     appends it to the level's candidate list, the candidates are sorted by
+//     key (CUB radix sort), candidate i gets new id hi + i, and the host reads
+//     one count.
 // Then the unreached vertices are appended in ascending id (CUB select), the
 // new row offsets are a scan of the permuted degrees, and one warp per new
-// row copies and renames its arcs.  Everything stays on the device; the
-// host reads one count per level.
+// row copies and renames its arcs.
 #include "host_graph.h"
 #include "mlmq_b200.h"
 #include "solver_internal.h"
 
+#include <cooperative_groups.h>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 #include <cub/device/device_select.cuh>
@@ -39,6 +51,8 @@
 namespace mlmq {
 namespace {
 
+namespace cg = cooperative_groups;
+
 constexpr unsigned long long NO_KEY = ~0ull;
 
 __global__ void reorder_init_kernel(int n, int *inv, unsigned long long *key, int *mark) {
@@ -49,9 +63,250 @@ __global__ void reorder_init_kernel(int n, int *inv, unsigned long long *key, in
     }
 }
 
-__global__ void reorder_seed_kernel(int root, int *inv, int *perm) {
+__global__ void reorder_seed_kernel(int root, int *inv, int *perm, unsigned long long *key) {
     inv[root] = 0;
     perm[0] = root;
+    key[root] = 0ull;  // below every proposal
+}
+
+constexpr int NARROW_THREADS = 1024;
+constexpr int NARROW_CAP = NARROW_THREADS;  // vertices of a level in one CTA
+constexpr int NARROW_DEGREE = 32;           // arcs of a vertex, below a bit each
+constexpr int NARROW_LEVELS = 1 << 16;      // levels of one launch, so that each is bounded
+constexpr int MIDDLE_CTAS = 8, MIDDLE_THREADS = 512, MIDDLE_ROUNDS = 3;
+constexpr int MIDDLE_CAP = MIDDLE_CTAS * MIDDLE_THREADS * MIDDLE_ROUNDS;
+// The cluster hands a level below this back to the one CTA, which keeps it up
+// to NARROW_CAP: the gap keeps the two from taking turns.
+constexpr int MIDDLE_MIN = 512;
+
+// A frontier vertex: id, first arc, degree.  The proposals of one thread's
+// vertex at queue position `pos`; `won` gets the arcs that still stand, t the
+// first four targets, their rows loaded beside the atomics.
+__device__ __forceinline__ void reorder_propose(const int *__restrict__ row, const int *__restrict__ col,
+                                                unsigned long long *key, int3 u, int pos, unsigned &won,
+                                                int3 (&t)[4]) {
+    const unsigned long long k = (unsigned long long)pos << 32;
+    won = 0u;
+    for (int j0 = 0; j0 < u.z; j0 += 4) {
+        int v[4], beg[4], end[4];
+        unsigned long long was[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) v[q] = j0 + q < u.z ? __ldg(col + u.y + j0 + q) : -1;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            was[q] = 0ull;
+            beg[q] = end[q] = 0;
+            if (v[q] < 0) continue;
+            was[q] = atomicMin(key + v[q], k | (unsigned)(j0 + q));
+            if (j0 == 0) {
+                beg[q] = __ldg(row + v[q]);
+                end[q] = __ldg(row + v[q] + 1);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (was[q] > (k | (unsigned)(j0 + q))) won |= 1u << (j0 + q);
+            if (j0 == 0) t[q] = make_int3(v[q], beg[q], end[q] - beg[q]);
+        }
+    }
+}
+
+// Of the arcs in `won`, those whose key stands now that every proposal is in.
+__device__ __forceinline__ unsigned reorder_check(const int *__restrict__ col,
+                                                  const unsigned long long *key, int3 u, int pos,
+                                                  unsigned won, const int3 (&t)[4]) {
+    const unsigned long long k = (unsigned long long)pos << 32;
+    unsigned wins = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        if ((won >> q) & 1u && __ldcg(key + t[q].x) == (k | (unsigned)q)) wins |= 1u << q;
+    for (unsigned rest = won & ~15u; rest; rest &= rest - 1u) {
+        const int j = __ffs(rest) - 1;
+        if (__ldcg(key + __ldg(col + u.y + j)) == (k | (unsigned)j)) wins |= 1u << j;
+    }
+    return wins;
+}
+
+// Target j of a vertex as a frontier vertex.
+__device__ __forceinline__ int3 reorder_target(const int *__restrict__ row, const int *__restrict__ col,
+                                               int3 u, int j, const int3 (&t)[4]) {
+    if (j < 4) return j == 0 ? t[0] : j == 1 ? t[1] : j == 2 ? t[2] : t[3];
+    const int v = __ldg(col + u.y + j), beg = __ldg(row + v);
+    return make_int3(v, beg, __ldg(row + v + 1) - beg);
+}
+
+// Exclusive prefix sum of `mine` over the CTA's threads and the total; `sums`
+// holds one int per warp.  Ends with every thread past its reads of `sums`.
+__device__ __forceinline__ int reorder_scan(int mine, int *sums, int *total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    int incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += x;
+    }
+    if (lane == 31) sums[warp] = incl;
+    __syncthreads();
+    const int own = lane < warps ? sums[lane] : 0;
+    int x = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    *total = __shfl_sync(0xffffffffu, x, 31);
+    const int before = __shfl_sync(0xffffffffu, x - own, warp);
+    __syncthreads();
+    return before + incl - mine;
+}
+
+// Levels from queue positions [state[0], state[1]) on, by one CTA, until one is
+// empty or not narrow, or NARROW_LEVELS are done; state becomes the level to
+// go on with.
+__global__ void __launch_bounds__(NARROW_THREADS, 1)
+    reorder_narrow_kernel(const int *__restrict__ row, const int *__restrict__ col, int *perm, int *inv,
+                          unsigned long long *key, int *state) {
+    __shared__ int3 list[2][NARROW_CAP];
+    __shared__ int sums[NARROW_THREADS / 32];
+    const int tid = threadIdx.x;
+    int lo = state[0], hi = state[1], half = 0;
+    if (hi - lo <= NARROW_CAP && tid < hi - lo) {
+        const int u = perm[lo + tid], beg = row[u];
+        list[0][tid] = make_int3(u, beg, row[u + 1] - beg);
+    }
+    for (int level = 0; level < NARROW_LEVELS; level++, half ^= 1) {
+        const int size = hi - lo;
+        if (size <= 0 || size > NARROW_CAP) break;
+        // (The barrier also covers the list.)
+        __syncthreads();
+        const int3 u = tid < size ? list[half][tid] : make_int3(0, 0, 0);
+        if (__syncthreads_or(u.z > NARROW_DEGREE)) break;
+        unsigned won;
+        int3 t[4];
+        reorder_propose(row, col, key, u, lo + tid, won, t);
+        __syncthreads();
+        unsigned wins = reorder_check(col, key, u, lo + tid, won, t);
+        int found;
+        int at = reorder_scan(__popc(wins), sums, &found);
+        for (; wins; wins &= wins - 1u, at++) {
+            const int3 v = reorder_target(row, col, u, __ffs(wins) - 1, t);
+            perm[hi + at] = v.x;
+            inv[v.x] = hi + at;
+            if (at < NARROW_CAP) list[half ^ 1][at] = v;
+        }
+        lo = hi;
+        hi += found;
+    }
+    if (tid == 0) {
+        state[0] = lo;
+        state[1] = hi;
+    }
+}
+
+// The same by a cluster: queue positions go to the CTAs in blocks of
+// MIDDLE_THREADS in turn, so a thread's vertices of a level are MIDDLE_ROUNDS
+// at most; a found vertex goes straight to its next thread's place in that
+// CTA's shared memory.
+__global__ void __cluster_dims__(MIDDLE_CTAS, 1, 1) __launch_bounds__(MIDDLE_THREADS, 1)
+    reorder_middle_kernel(const int *__restrict__ row, const int *__restrict__ col, int *perm, int *inv,
+                          unsigned long long *key, int *state) {
+    __shared__ int3 list[2][MIDDLE_ROUNDS * MIDDLE_THREADS];
+    __shared__ int counts[2][MIDDLE_ROUNDS][MIDDLE_CTAS];  // found by round and CTA, by level parity
+    __shared__ int big[2];                                 // by level parity
+    __shared__ int sums[MIDDLE_THREADS / 32];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int tid = threadIdx.x, rank = (int)cluster.block_rank();
+    int lo = state[0], hi = state[1], half = 0;
+    if (tid < 2) big[tid] = 0;
+    if (hi - lo <= MIDDLE_CAP)
+        for (int r = 0; r < MIDDLE_ROUNDS; r++) {
+            const int i = (r * MIDDLE_CTAS + rank) * MIDDLE_THREADS + tid;
+            if (i < hi - lo) {
+                const int u = perm[lo + i], beg = row[u];
+                const int3 e = make_int3(u, beg, row[u + 1] - beg);
+                list[0][r * MIDDLE_THREADS + tid] = e;
+                if (e.z > NARROW_DEGREE)
+                    for (int c = 0; c < MIDDLE_CTAS; c++) *cluster.map_shared_rank(&big[0], c) = 1;
+            }
+        }
+    // Every CTA has read the state and set its flags before any is written.
+    cluster.sync();
+    for (int level = 0; level < NARROW_LEVELS; level++, half ^= 1) {
+        const int size = hi - lo;
+        if (size <= 0 || size > MIDDLE_CAP || (level > 0 && size < MIDDLE_MIN) || big[half]) break;
+        unsigned won[MIDDLE_ROUNDS];
+        int3 t0[4], tr[4];
+#pragma unroll
+        for (int r = 0; r < MIDDLE_ROUNDS; r++) {
+            const int i = (r * MIDDLE_CTAS + rank) * MIDDLE_THREADS + tid;
+            won[r] = 0u;
+            if (i >= size) continue;
+            const int3 u = list[half][r * MIDDLE_THREADS + tid];
+            if (r == 0) reorder_propose(row, col, key, u, lo + i, won[r], t0);
+            else reorder_propose(row, col, key, u, lo + i, won[r], tr);
+        }
+        cluster.sync();
+        int at[MIDDLE_ROUNDS];
+#pragma unroll
+        for (int r = 0; r < MIDDLE_ROUNDS; r++) {
+            const int i = (r * MIDDLE_CTAS + rank) * MIDDLE_THREADS + tid;
+            at[r] = 0;
+            int found = 0;
+            if (r * MIDDLE_CTAS * MIDDLE_THREADS < size) {
+                if (i < size && won[r]) {
+                    const int3 u = list[half][r * MIDDLE_THREADS + tid];
+                    if (r > 0)
+                        for (int q = 0; q < 4; q++) tr[q].x = q < u.z ? __ldg(col + u.y + q) : -1;
+                    won[r] = r == 0 ? reorder_check(col, key, u, lo + i, won[r], t0)
+                                    : reorder_check(col, key, u, lo + i, won[r], tr);
+                }
+                at[r] = reorder_scan(__popc(won[r]), sums, &found);
+            }
+            if (tid < MIDDLE_CTAS) *cluster.map_shared_rank(&counts[half][r][rank], tid) = found;
+        }
+        if (tid == 0) big[half] = 0;  // of the level after next
+        cluster.sync();
+        int all = 0;
+#pragma unroll
+        for (int r = 0; r < MIDDLE_ROUNDS; r++) {
+            const int i = (r * MIDDLE_CTAS + rank) * MIDDLE_THREADS + tid;
+            int before = all;
+            for (int c = 0; c < MIDDLE_CTAS; c++) {
+                const int x = counts[half][r][c];
+                if (c < rank) before += x;
+                all += x;
+            }
+            int to = before + at[r];
+            const int3 u = i < size && won[r] ? list[half][r * MIDDLE_THREADS + tid] : make_int3(0, 0, 0);
+            for (unsigned wins = won[r]; wins; wins &= wins - 1u, to++) {
+                int3 v;
+                const int j = __ffs(wins) - 1;
+                if (r == 0) {
+                    v = reorder_target(row, col, u, j, t0);
+                } else {
+                    v.x = __ldg(col + u.y + j);
+                    v.y = __ldg(row + v.x);
+                    v.z = __ldg(row + v.x + 1) - v.y;
+                }
+                perm[hi + to] = v.x;
+                inv[v.x] = hi + to;
+                if (to < MIDDLE_CAP) {
+                    const int block = to / MIDDLE_THREADS;
+                    const int place = block / MIDDLE_CTAS * MIDDLE_THREADS + to % MIDDLE_THREADS;
+                    *cluster.map_shared_rank(&list[half ^ 1][place], block % MIDDLE_CTAS) = v;
+                }
+                if (v.z > NARROW_DEGREE)
+                    for (int c = 0; c < MIDDLE_CTAS; c++) *cluster.map_shared_rank(&big[half ^ 1], c) = 1;
+            }
+        }
+        lo = hi;
+        hi += all;
+        cluster.sync();
+    }
+    if (rank == 0 && tid == 0) {
+        state[0] = lo;
+        state[1] = hi;
+    }
 }
 
 // One warp per vertex of the current level: its lanes stride the row.
@@ -76,11 +331,10 @@ __global__ void reorder_discover_kernel(const int *__restrict__ row, const int *
 }
 
 __global__ void reorder_gather_keys_kernel(const int *__restrict__ cand, int c,
-                                           unsigned long long *key, unsigned long long *ck) {
+                                           const unsigned long long *key, unsigned long long *ck) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < c; i += gridDim.x * blockDim.x) {
         const int v = cand[i];
-        ck[i] = key[v];
-        key[v] = NO_KEY;
+        ck[i] = key[v];  // stays: below every later proposal
     }
 }
 
@@ -179,11 +433,34 @@ extern "C" int mlmq_reorder_bfs_device(int n, int64_t m, const int *d_row, const
     }
     if (!rc) {
         reorder_init_kernel<<<grid_for(n, 256), 256, 0, st>>>(n, inv, key, mark);
-        reorder_seed_kernel<<<1, 1, 0, st>>>(root, inv, perm);
+        reorder_seed_kernel<<<1, 1, 0, st>>>(root, inv, perm, key);
         rc = cuda_fail(cudaGetLastError(), "reorder init");
     }
     int lo = 0, hi = 1;
     for (int level = 0; !rc && lo < hi; level++) {
+        // Narrow levels up to the next wide one, by one CTA or a cluster.
+        bool wide = hi - lo > MIDDLE_CAP;
+        while (!rc && !wide && lo < hi) {
+            const int before = lo;
+            const bool one = hi - lo <= NARROW_CAP;
+            h_count[0] = lo;
+            h_count[1] = hi;
+            rc = cuda_fail(cudaMemcpyAsync(count, h_count, 2 * sizeof(int), cudaMemcpyHostToDevice, st),
+                           "reorder level");
+            if (!rc) {
+                if (one) reorder_narrow_kernel<<<1, NARROW_THREADS, 0, st>>>(d_row, d_col, perm, inv, key, count);
+                else reorder_middle_kernel<<<MIDDLE_CTAS, MIDDLE_THREADS, 0, st>>>(d_row, d_col, perm, inv, key, count);
+                rc = cuda_fail(cudaGetLastError(), "reorder narrow levels");
+            }
+            if (!rc) rc = cuda_fail(cudaMemcpyAsync(h_count, count, 2 * sizeof(int), cudaMemcpyDeviceToHost,
+                                                    st), "reorder level");
+            if (!rc) rc = cuda_fail(cudaStreamSynchronize(st), "reorder level");
+            if (rc) break;
+            lo = h_count[0];
+            hi = h_count[1];
+            wide = lo == before || hi - lo > MIDDLE_CAP;  // no level done: a vertex of many arcs
+        }
+        if (rc || lo >= hi) break;
         rc = cuda_fail(cudaMemsetAsync(count, 0, sizeof(int), st), "reorder count reset");
         if (rc) break;
         reorder_discover_kernel<<<grid_for((long long)(hi - lo) * 32, 256), 256, 0, st>>>(

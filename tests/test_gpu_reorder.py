@@ -1,0 +1,56 @@
+"""The device reordering at the edges between its narrow levels (one CTA, a
+vertex per thread) and its wide ones: byte-identical to the host search."""
+import numpy as np
+import pytest
+
+from mlmq_tpds_withl3_b200 import HostGraph
+
+pytestmark = pytest.mark.gpu
+
+
+def _layers(sizes, degree, seed):
+    """Layer k's vertices, in shuffled ids, reach all of layer k + 1; each has
+    `degree` arcs at most, the others to random vertices of earlier layers, its
+    own and the next (duplicates and self loops among them)."""
+    rng = np.random.default_rng(seed)
+    n = sum(sizes) + 5  # 5 vertices that the search never reaches
+    ids = rng.permutation(n)
+    adj = [[] for _ in range(n)]
+    base = 0
+    for k, size in enumerate(sizes):
+        nxt = sizes[k + 1] if k + 1 < len(sizes) else 0
+        for i in range(nxt):
+            adj[base + i % size].append(base + size + i)
+        for i in range(size):
+            more = degree - len(adj[base + i])
+            if more > 0:
+                adj[base + i] += rng.integers(max(0, base - 50), base + size + nxt, more).tolist()
+        base += size
+    src = np.repeat(np.arange(n), [len(a) for a in adj])
+    dst = np.concatenate([np.asarray(a, np.int64) for a in adj if a])
+    order = np.argsort(ids[src], kind="stable")
+    row = np.zeros(n + 1, np.int64)
+    row[1:] = np.cumsum(np.bincount(ids[src], minlength=n))
+    g = HostGraph.from_csr(row, ids[dst][order], np.arange(len(dst)) % 97 + 1, "layers")
+    return g, int(ids[0])
+
+
+@pytest.mark.parametrize("sizes,degree", [
+    ([1], 1), ([1, 31, 1023, 1024, 1025, 3], 8), ([1, 32, 1024, 8191, 8192, 8193, 1, 2], 12),
+    ([1, 32, 1024, 30000, 40, 20000, 700], 30),
+    ([1, 30, 511, 512, 513, 1025, 4096, 4097, 511, 1500, 12288, 9000, 12289, 1030, 5], 20),
+    ([1, 30, 900, 1100, 1100, 1100, 600], 32), ([1, 30, 900, 1100, 1100, 1100, 600], 33), ([1, 32, 500, 900], 32), ([1, 33, 500, 900], 33)])
+def test_levels_at_the_edges(sizes, degree):
+    g, root = _layers(sizes, degree, sum(sizes))
+    want, got = g.reorder_bfs(root), g.reorder_bfs_gpu(root)
+    for a, b in zip(want[1:], got[1:]):
+        assert np.array_equal(a, b)
+    for name in ("row", "col", "w"):
+        assert np.array_equal(getattr(want[0], name), getattr(got[0], name)), name
+
+
+def test_more_levels_than_one_launch_runs():
+    n = (1 << 16) + 300
+    row = np.minimum(np.arange(n + 1), n - 1)
+    g = HostGraph.from_csr(row, np.arange(1, n), np.ones(n - 1), "path")
+    assert np.array_equal(g.reorder_bfs(7)[1], g.reorder_bfs_gpu(7)[1])
