@@ -77,10 +77,23 @@ struct PlainParams {
     const int *__restrict__ split;  // light arcs (w < delta) per vertex, or null: no split
     int precheck;  // read dist[dst] before the atomicMin
     unsigned delta;
+    unsigned delta_inv, nb_inv;  // quotient_inverse of delta and nb
     int l2_log, l3_log;
     int workers;  // worker warps per CTA (one more warp per CTA is the manager)
     unsigned long long timeout_ns;
 };
+
+// floor((2^32 - 1) / y), for quotients by a divisor that is fixed for a solve.
+__host__ __device__ __forceinline__ unsigned quotient_inverse(unsigned y) { return 0xffffffffu / y; }
+// x / y with y's inverse: the high product is the quotient or one less (its
+// error is below x (1 + 1/y) / 2^32 plus the truncation, so below 2 for any x
+// below 2^32).  A runtime division is a chain of some twenty instructions, and
+// a push, a read and an idle poll had one to three of them each.
+__device__ __forceinline__ unsigned quotient(unsigned x, unsigned y, unsigned inv) {
+    unsigned q = __umulhi(x, inv);
+    if (x - q * y >= y) q++;
+    return q;
+}
 
 // Shared-memory copy of the global queue counters, refreshed by the manager
 // warp of each CTA.
@@ -183,13 +196,13 @@ __device__ __forceinline__ void push32(const PlainParams &p, WarpQ &q, bool vali
     const unsigned upres = m.u_pressure;
     int tgt = -1;
     if (valid) {
-        const unsigned L = d / p.delta;
+        const unsigned L = quotient(d, p.delta, p.delta_inv);
         if (L < f) {
             tgt = upres ? NB_MAX : p.nb;  // urgent ring, or L3 while it is filling
         } else if (L - f >= (unsigned)p.nb) {
             tgt = NB_MAX;  // L3
         } else {
-            const int b = (int)(L % (unsigned)p.nb);
+            const int b = (int)(L - quotient(L, (unsigned)p.nb, p.nb_inv) * (unsigned)p.nb);
             tgt = ((pres >> b) & 1u) ? NB_MAX : b;
         }
     }
@@ -417,9 +430,10 @@ __device__ __forceinline__ bool l2_has_work(const PlainParams &p, const WarpQ &q
     const int lane = threadIdx.x & 31;
     bool has = false;
     if (lane <= p.nb) {
-        const unsigned rel = ((unsigned)lane + (unsigned)p.nb - mir.first % (unsigned)p.nb) %
-                             (unsigned)p.nb;
-        if (lane == p.nb || rel < (unsigned)p.bm) {
+        const unsigned f = mir.first;
+        int rel = lane - (int)(f - quotient(f, (unsigned)p.nb, p.nb_inv) * (unsigned)p.nb);
+        if (rel < 0) rel += p.nb;
+        if (lane == p.nb || rel < p.bm) {
             const unsigned res = mir.reserve[lane];
             has = (int)(res - mir.claim[lane]) > 0 || (q.c_lo != q.c_hi && res != q.c_lo);
         }
@@ -434,9 +448,10 @@ __device__ __forceinline__ int l2_read(const PlainParams &p, WarpQ &q, volatile 
                                        uint2 *inb, int room, int want) {
     int got = read_ring(p, q, mir, p.nb, inb, 0, room);
     const unsigned f = mir.first;
+    int b = (int)(f - quotient(f, (unsigned)p.nb, p.nb_inv) * (unsigned)p.nb);
     for (int i = 0; i < p.bm && got < want; i++) {
-        const int b = (int)((f + (unsigned)i) % (unsigned)p.nb);
         got += read_ring(p, q, mir, b, inb, got, room);
+        if (++b == p.nb) b = 0;
     }
     return got;
 }

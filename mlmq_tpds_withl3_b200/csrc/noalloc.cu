@@ -204,6 +204,8 @@ extern "C" int mlmq_sssp_solve_noalloc(int n, int m, const int *d_row, const int
     p.split = nullptr;  // the light/heavy split needs vertex tiles
     p.precheck = cfg.relax_precheck;
     p.delta = (unsigned)cfg.delta;
+    p.delta_inv = quotient_inverse(p.delta);
+    p.nb_inv = quotient_inverse((unsigned)p.nb);
     p.l2_log = NA_L2_LOG;
     p.l3_log = NA_L3_LOG;
     p.workers = workers;

@@ -1074,6 +1074,8 @@ extern "C" int mlmq_solver_launch(mlmq_solver *s, int src, void *stream) {
     p.split = s->split;
     p.precheck = s->cfg.relax_precheck;
     p.delta = (unsigned)s->cfg.delta;
+    p.delta_inv = quotient_inverse(p.delta);
+    p.nb_inv = quotient_inverse((unsigned)p.nb);
     p.l2_log = s->l2_log;
     p.l3_log = s->l3_log;
     p.workers = s->workers;

@@ -180,6 +180,8 @@ int enqueue(mlmq_batch *b, int nq, cudaStream_t st) {
     p.split = nullptr;  // per query
     p.precheck = b->cfg.relax_precheck;
     p.delta = (unsigned)b->cfg.delta;
+    p.delta_inv = quotient_inverse(p.delta);
+    p.nb_inv = quotient_inverse((unsigned)p.nb);
     p.l2_log = b->l2_log;
     p.l3_log = b->l3_log;
     p.workers = b->workers;

@@ -85,7 +85,7 @@ __device__ __forceinline__ void manager_loop(const PlainParams &p, volatile Mirr
                 // to the smallest distance pushed to L3 since the last one.
                 if (lane == 0) {
                     const unsigned m = atomicExch(p.ctlw + ctl::L3_MIN, 0xffffffffu);
-                    if (m != 0xffffffffu) atomicMax(p.ctlw + ctl::FIRST, m / p.delta);
+                    if (m != 0xffffffffu) atomicMax(p.ctlw + ctl::FIRST, quotient(m, p.delta, p.delta_inv));
                     st_release(p.ctlw + ctl::L3_EPOCH, l3r);
                 }
             } else {
@@ -98,7 +98,8 @@ __device__ __forceinline__ void manager_loop(const PlainParams &p, volatile Mirr
                     // producing records in warps' L1 rings, and a window that
                     // runs ahead of them turns their results into urgent
                     // corrections of work already done.
-                    const int b = (int)((first + (unsigned)lane) % (unsigned)p.nb);
+                    const unsigned at = first + (unsigned)lane;
+                    const int b = (int)(at - quotient(at, (unsigned)p.nb, p.nb_inv) * (unsigned)p.nb);
                     const unsigned rb = __shfl_sync(FULL, res, b);
                     const unsigned cb = __shfl_sync(FULL, con, b);
                     const unsigned ne = __ballot_sync(FULL, lane < p.nb && rb != cb);

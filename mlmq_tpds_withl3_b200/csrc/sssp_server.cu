@@ -274,6 +274,7 @@ __global__ void __maxnreg__(SLOT_KERNEL_REGS) sssp_server_kernel(ServerParams sp
             p.arcs = (const int2 *)(((unsigned long long)cmd[3] << 32) | cmd[2]);
             p.tiles = (const int4 *)(((unsigned long long)cmd[7] << 32) | cmd[6]);
             p.delta = cmd[8];
+            p.delta_inv = quotient_inverse(p.delta);
             p.topup = (int)cmd[9];
             p.l1_ahead = (int)cmd[10];
             p.bm = (int)cmd[11];
@@ -552,6 +553,8 @@ int server_create(int slots, const int *layout, int max_vertices, const mlmq_con
         b.split = nullptr;  // per query
         b.precheck = cfg.relax_precheck;
         b.delta = (unsigned)cfg.delta;
+        b.delta_inv = quotient_inverse(b.delta);
+        b.nb_inv = quotient_inverse((unsigned)b.nb);
         b.l2_log = sv->l2_log;
         b.l3_log = sv->l3_log;
         b.workers = sv->workers;
