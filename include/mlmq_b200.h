@@ -423,8 +423,8 @@ void mlmq_server_destroy(mlmq_server *sv);
  * place) and the output d_dist[n]; nothing else is allocated.
  *
  *  - Graphs above MLMQ_NOALLOC_MAX_VERTICES vertices or MLMQ_NOALLOC_MAX_ARCS
- *    arcs, and bucket_num > 16, return MLMQ_ERR_RANGE before any work; at
- *    most 8 worker warps per CTA are used.
+ *    arcs, and bucket_num > 16, return MLMQ_ERR_RANGE before any work; the
+ *    asynchronous kernel uses at most 8 worker warps per CTA.
  *  - cfg may be NULL (mlmq_config_default).  The call runs on `stream`
  *    (a cudaStream_t, NULL = legacy default stream) and returns when the
  *    solve has finished, with its status.

@@ -36,6 +36,7 @@
 #include "sssp_plain.h"
 #include "sssp_plain_body.cuh"
 
+#include <algorithm>
 #include <cstdio>
 #include <mutex>
 
@@ -61,6 +62,32 @@ static __device__ __align__(256) unsigned long long g_noalloc_ws[NA_TOTAL_U64];
 // Relaxes one round of 32 arcs at a time (relax_unroll does not apply here).
 __global__ void __launch_bounds__(1024, 1) sssp_noalloc_kernel(PlainParams p) {
     plain_body<ArcsSplit, 1>(p, blockIdx.x, gridDim.x);
+}
+
+// What the choice of kernel needs to know of the caller's CSR: out[0] largest
+// degree, out[1] of a sample of arcs those that leave their tail's block of
+// consecutive vertices, out[2] all of the sample.
+__global__ void shape_kernel(const int *__restrict__ row, const int *__restrict__ col, int n, unsigned block,
+                             unsigned *out) {
+    int degree = 0;
+    unsigned away = 0, all = 0;
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+        const int beg = row[v], deg = row[v + 1] - beg;
+        degree = max(degree, deg);
+        if ((v & 7) != 0) continue;
+        for (int i = 0; i < min(deg, 8); i++) {
+            away += (unsigned)col[beg + i] / block != (unsigned)v / block;
+            all++;
+        }
+    }
+    degree = __reduce_max_sync(FULL, degree);
+    away = __reduce_add_sync(FULL, away);
+    all = __reduce_add_sync(FULL, all);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(out, (unsigned)degree);
+        atomicAdd(out + 1, away);
+        atomicAdd(out + 2, all);
+    }
 }
 
 struct DeviceSlot {
@@ -222,12 +249,46 @@ extern "C" int mlmq_sssp_solve_noalloc(int n, int m, const int *d_row, const int
     lc.attrs = attr;
     lc.numAttrs = 1;
     slot->clean = false;
-    rc = cuda_fail(cudaLaunchKernelEx(&lc, sssp_noalloc_kernel, p), "no-alloc launch");
-    if (rc) return rc;
+    // The vertex-owner kernel where the CSR's shape suits it (its rule takes
+    // one more launch and a copy, about 15 us).  Its inbox tails take the place
+    // of the L3 bits, which every solve that uses them clears first.
+    int ctas = 0, block = 0;
+    if (cfg.queue_type == MLMQ_L1SLF_L2DQ && !cfg.bucket_sync) block = owner_block(n, sms, &ctas);
+    if (block && (cfg.work_blocks == 0 || ctas <= cfg.work_blocks)) {
+        unsigned *d_shape = p.ctlw + ctl::WORDS, shape[3] = {0, 0, 0};
+        rc = cuda_fail(cudaMemsetAsync(d_shape, 0, sizeof(shape), st), "shape");
+        if (rc) return rc;
+        shape_kernel<<<std::min((n + 255) / 256, sms * 4), 256, 0, st>>>(d_row, d_col, n, (unsigned)block, d_shape);
+        rc = cuda_fail(cudaGetLastError(), "shape launch");
+        if (!rc) rc = cuda_fail(cudaMemcpyAsync(shape, d_shape, sizeof(shape), cudaMemcpyDeviceToHost, st),
+                                "shape copy");
+        if (!rc) rc = cuda_fail(cudaStreamSynchronize(st), "shape");
+        if (rc) return rc;
+        const float away = shape[2] ? (float)shape[1] / (float)shape[2] : 1.0f;
+        if (!owner_fits(n, m, (int)shape[0], away, ctas, p.nb + 1, p.l2_log)) block = 0;
+    } else {
+        block = 0;
+    }
     unsigned status = 0;
-    rc = cuda_fail(cudaMemcpyAsync(&status, p.ctlw + ctl::STATUS, sizeof(status),
-                                   cudaMemcpyDeviceToHost, st), "status copy");
-    if (!rc) rc = cuda_fail(cudaStreamSynchronize(st), "no-alloc solve");
+    if (block) {
+        rc = cuda_fail(owner_prepare(), "owner shared memory");
+        if (!rc) rc = cuda_fail(owner_launch(p, block, ctas, l3bits, st), "no-alloc launch");
+        if (!rc) rc = cuda_fail(cudaMemcpyAsync(&status, p.ctlw + ctl::STATUS, sizeof(status),
+                                                cudaMemcpyDeviceToHost, st), "status copy");
+        if (!rc) rc = cuda_fail(cudaStreamSynchronize(st), "no-alloc solve");
+        if (!rc && (status & ST_QUEUE_FULL)) {
+            // Inboxes that filled each other up: the asynchronous kernel.
+            block = 0;
+            rc = cuda_fail(cudaMemsetAsync(ctl_base, 0, NA_CTL_U64 * 8, st), "clear control");
+            if (!rc) rc = cuda_fail(cudaMemsetAsync(l2, 0xff, (NA_L2_U64 + NA_L3_U64) * 8, st), "clear rings");
+        }
+    }
+    if (!rc && !block) {
+        rc = cuda_fail(cudaLaunchKernelEx(&lc, sssp_noalloc_kernel, p), "no-alloc launch");
+        if (!rc) rc = cuda_fail(cudaMemcpyAsync(&status, p.ctlw + ctl::STATUS, sizeof(status),
+                                                cudaMemcpyDeviceToHost, st), "status copy");
+        if (!rc) rc = cuda_fail(cudaStreamSynchronize(st), "no-alloc solve");
+    }
     if (rc) return rc;
     rc = status_to_error(status);
     // A finished solve consumed every record it reserved: the rings are empty.

@@ -955,18 +955,14 @@ extern "C" int mlmq_solver_create(const mlmq_graph *g, const mlmq_config *cfg_in
         mlmq_solver_destroy(s);
         return rc;
     }
-    // Vertices in a local order, none of many arcs, an SLF queue without the
-    // split or synchronised buckets: the vertex-owner kernel.  Its wavefront
-    // hops inside an SM; with many arcs between blocks it would send messages
-    // instead, and a vertex of many arcs would hold up its CTA's ticks.  Above
-    // OWNER_MAX_N vertices its longer lists and tiles from HBM take as long as
-    // the asynchronous kernel's hops (3M points 6.2 ms on both).
-    constexpr int OWNER_MAX_N = 3 << 20, OWNER_MAX_DEGREE = 32;
+    // Vertices in a local order and an SLF queue without the split or
+    // synchronised buckets: the vertex-owner kernel.
     int owner_ctas = 0;
-    if (cfg.queue_type == MLMQ_L1SLF_L2DQ && !cfg.light_heavy && !cfg.bucket_sync &&
-        g->n <= OWNER_MAX_N && g->max_degree <= OWNER_MAX_DEGREE && g->away <= 0.125f) {
+    if (cfg.queue_type == MLMQ_L1SLF_L2DQ && !cfg.light_heavy && !cfg.bucket_sync) {
         const int block = owner_block(g->n, sms, &owner_ctas);
-        if (block && (cfg.work_blocks == 0 || owner_ctas <= cfg.work_blocks)) s->owner_block = block;
+        if (block && (cfg.work_blocks == 0 || owner_ctas <= cfg.work_blocks) &&
+            owner_fits(g->n, g->m, g->max_degree, g->away, owner_ctas, cfg.bucket_num + 1, s->l2_log))
+            s->owner_block = block;
     }
     if (s->owner_block) {
         rc = cuda_fail(owner_prepare(), "owner shared memory");
@@ -988,7 +984,7 @@ extern "C" int mlmq_solver_create(const mlmq_graph *g, const mlmq_config *cfg_in
         const int maxgrid = bps * sms;
         s->grid = cfg.work_blocks > 0 ? std::min(cfg.work_blocks, maxgrid) : sms;
         if (s->grid > maxgrid) s->grid = maxgrid;
-        if (s->owner_block) s->grid = owner_ctas;
+        s->owner_ctas = owner_ctas;
     }
     const size_t l2_bytes = sizeof(unsigned long long) * ((size_t)(cfg.bucket_num + 1) << s->l2_log);
     const size_t l3_bytes = sizeof(unsigned long long) * ((size_t)1 << s->l3_log);
@@ -1042,6 +1038,8 @@ extern "C" int mlmq_solver_launch(mlmq_solver *s, int src, void *stream) {
         }
     }
     cudaStream_t st = stream ? (cudaStream_t)stream : s->stream;
+    s->src = src;
+    s->last = st;
     int rc = MLMQ_OK;
     if (s->dirty && (rc = reset_workspace(s, st))) return rc;
     PlainParams p;
@@ -1081,7 +1079,7 @@ extern "C" int mlmq_solver_launch(mlmq_solver *s, int src, void *stream) {
     p.workers = s->workers;
     p.timeout_ns = (unsigned long long)s->cfg.timeout_ms * 1000000ull;
     rc = s->owner_block
-             ? cuda_fail(owner_launch(p, s->owner_block, s->grid, s->d_tails, st), "owner launch")
+             ? cuda_fail(owner_launch(p, s->owner_block, s->owner_ctas, s->d_tails, st), "owner launch")
              : cuda_fail(plain_launch(p, s->cfg.relax_unroll, s->grid, st), "persistent launch");
     if (rc) {
         s->dirty = true;
@@ -1107,6 +1105,13 @@ extern "C" int mlmq_solver_wait(mlmq_solver *s) {
     const unsigned st = s->h_ctl[ctl::STATUS];
     rc = status_to_error(st);
     if (rc && rc != MLMQ_ERR_RANGE) s->dirty = true;
+    if (rc == MLMQ_ERR_QUEUE_FULL && s->owner_block) {
+        // Inboxes that filled each other up: the asynchronous kernel, whose
+        // rings divert to L3, takes this solver from here on.
+        s->owner_block = 0;
+        rc = mlmq_solver_launch(s, s->src, s->last);
+        return rc ? rc : mlmq_solver_wait(s);
+    }
     return rc;
 }
 
@@ -1139,7 +1144,7 @@ extern "C" int mlmq_solver_stats(mlmq_solver *s, mlmq_solve_stats *st) {
     st->first_max = (uint32_t)c[ctl::ST_FIRST_MAX];
     st->batches = c[ctl::ST_BATCHES];
     st->idle = c[ctl::ST_IDLE];
-    st->grid = s->grid;
+    st->grid = s->owner_block ? s->owner_ctas : s->grid;
     st->block = s->owner_block ? owner_threads() : 32 * (s->workers + 1);
     st->status = s->h_ctl[ctl::STATUS];
     return MLMQ_OK;
@@ -1267,7 +1272,8 @@ int dropin_run(int src) {
     if (src < 0 || src >= g_graph->n) return MLMQ_ERR_ARG;
     const char *qname = cfg.queue_type == MLMQ_L1V_L2DQ ? "L1V_L2DQ" : "L1SLF_L2DQ";
     std::printf("MLMQ_B200_CONFIG workers=%d blocks=%d delta=%d queue=%s\n",
-                g_solver->owner_block ? owner_threads() : 32 * g_solver->workers, g_solver->grid, cfg.delta, qname);
+                g_solver->owner_block ? owner_threads() : 32 * g_solver->workers,
+                g_solver->owner_block ? g_solver->owner_ctas : g_solver->grid, cfg.delta, qname);
     const int warmups = env_int("BENCH_WARMUPS", 2, nullptr);
     const int repeats = env_int("BENCH_REPEATS", 3, nullptr);
     if (warmups < 0 || repeats < 1) return MLMQ_ERR_ARG;

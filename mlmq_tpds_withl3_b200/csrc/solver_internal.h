@@ -55,6 +55,9 @@ struct mlmq_solver {
     unsigned *d_l3bits = nullptr;  // one bit per vertex: the vertex has an L3 record
     unsigned *d_ctl = nullptr;
     int owner_block = 0;        // vertices per CTA of the vertex-owner kernel; 0: not used
+    int owner_ctas = 0;
+    int src = 0;                // of the last launch, and its stream
+    cudaStream_t last = nullptr;
     unsigned *d_tails = nullptr; // its inbox tails, a line per CTA
     unsigned *h_ctl = nullptr;  // pinned copy of the control block after each solve
     cudaStream_t stream = nullptr;

@@ -9,13 +9,25 @@ namespace mlmq {
 // LPV lanes per vertex: 2 for 32-byte tiles and row offsets, 4 for 64-byte tiles.
 template <class Arcs, int LPV>
 __global__ void __launch_bounds__(OWNER_THREADS, 1) sssp_owner_kernel(PlainParams p, OwnerParams o) {
+    o.rank = blockIdx.x;
+    o.size = gridDim.x;
     owner_solve<Arcs, LPV>(p, o);
 }
 
 namespace {
-const void *owner_kernel(int tile_stride) {
+// The caller's separate arrays (no arc array) are read in place.
+const void *owner_kernel(int tile_stride, bool in_place) {
+    if (in_place) return (const void *)sssp_owner_kernel<ArcsSplit, 2>;
     return tile_stride == 4 ? (const void *)sssp_owner_kernel<ArcsInterleaved, 4>
                             : (const void *)sssp_owner_kernel<ArcsInterleaved, 2>;
+}
+
+// log2 slots of each of `ctas` inboxes in the memory of the L2 rings.
+int inbox_log(int ctas, int rings, int l2_log) {
+    const size_t slots = (size_t)rings << l2_log;
+    int log = 0;
+    while (log < 20 && ((size_t)ctas << (log + 1)) <= slots) log++;
+    return log;
 }
 }  // namespace
 
@@ -35,10 +47,26 @@ int owner_block(int n, int sms, int *ctas) {
 
 size_t owner_tails_bytes(int ctas) { return 128 * (size_t)ctas; }
 
+// Vertices in a local order, none of many arcs: the wavefront then hops inside
+// an SM (with many arcs between blocks it would send messages instead, and a
+// vertex of many arcs would hold up its CTA's ticks).  Above OWNER_MAX_N
+// vertices its longer lists and tiles from HBM take as long as the asynchronous
+// kernel's hops (3M points 6.2 ms on both, 6.3M points 8.0 against 7.9).  Each
+// inbox must hold its share of the arcs between blocks several times over, so
+// that a full one is out of the question in practice.
+int owner_fits(int n, int64_t m, int max_degree, float away, int ctas, int rings, int l2_log) {
+    constexpr int OWNER_MAX_N = 3 << 20, OWNER_MAX_DEGREE = 32;
+    if (n > OWNER_MAX_N || max_degree > OWNER_MAX_DEGREE) return 0;
+    if (ctas == 1) return 1;
+    return away <= 0.125f &&
+           4.0 * (double)away * (double)m / ctas + 1024.0 <= (double)(1 << inbox_log(ctas, rings, l2_log));
+}
+
 cudaError_t owner_prepare() {
-    for (int stride : {2, 4}) {
+    for (int k = 0; k < 3; k++) {
         const cudaError_t e =
-            cudaFuncSetAttribute(owner_kernel(stride), cudaFuncAttributeMaxDynamicSharedMemorySize,
+            cudaFuncSetAttribute(owner_kernel(k == 1 ? 4 : 2, k == 2),
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)owner_smem_bytes(OWNER_MAX_BLOCK));
         if (e != cudaSuccess) return e;
     }
@@ -53,9 +81,9 @@ cudaError_t owner_launch(const PlainParams &p, int block, int ctas, unsigned *ta
     o.tails = tails;
     // The inboxes share the memory of the L2 rings, which both kernels leave
     // empty.
-    const size_t slots = (size_t)(p.nb + 1) << p.l2_log;
-    o.inbox_log = 0;
-    while (o.inbox_log < 20 && ((size_t)ctas << (o.inbox_log + 1)) <= slots) o.inbox_log++;
+    o.inbox_log = inbox_log(ctas, p.nb + 1, p.l2_log);
+    o.rank = 0;
+    o.size = (unsigned)ctas;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3(OWNER_THREADS);
@@ -67,7 +95,7 @@ cudaError_t owner_launch(const PlainParams &p, int block, int ctas, unsigned *ta
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     void *args[] = {const_cast<PlainParams *>(&p), &o};
-    return cudaLaunchKernelExC(&cfg, owner_kernel(p.tile_stride), args);
+    return cudaLaunchKernelExC(&cfg, owner_kernel(p.tile_stride, p.col != nullptr), args);
 }
 
 }  // namespace mlmq

@@ -71,6 +71,7 @@ struct OwnerParams {
     unsigned block, block_inv;  // vertices per CTA (a multiple of 32), (2^32 - 1) / block
     int inbox_log;              // log2 slots of one inbox ring
     unsigned *tails;            // [CTAs] one 128-byte line each
+    unsigned rank, size;        // this CTA among the solve's
 };
 
 // Shared memory: distances, near bits, far bits, near lists, far lists.
@@ -498,7 +499,7 @@ __device__ __forceinline__ void owner_sender(const PlainParams &p, const OwnerPa
 __device__ __forceinline__ void owner_receiver(const PlainParams &p, const OwnerParams &o,
                                                OwnerShared &sh, unsigned long long *in) {
     const unsigned lane = threadIdx.x & 31u;
-    unsigned long long *ring = p.l2 + ((size_t)blockIdx.x << o.inbox_log);
+    unsigned long long *ring = p.l2 + ((size_t)o.rank << o.inbox_log);
     const unsigned mask = (1u << o.inbox_log) - 1u;
     unsigned at = 0;
     for (;;) {
@@ -540,7 +541,7 @@ __device__ __forceinline__ void owner_controller(const PlainParams &p, const Own
         const unsigned credit = ld_acquire(p.ctlw + ctl::CREDIT);
         __syncwarp();
         unsigned sum = 0;
-        for (unsigned c = lane; c < gridDim.x; c += 32) sum += ld_relaxed(o.tails + 32u * c);
+        for (unsigned c = lane; c < o.size; c += 32) sum += ld_relaxed(o.tails + 32u * c);
         sum = __reduce_add_sync(FULL, sum);
         if (sum == __shfl_sync(FULL, credit, 0)) {
             if (lane == 0) {
@@ -564,7 +565,7 @@ __device__ __forceinline__ void owner_solve(const PlainParams &p, const OwnerPar
     const unsigned tid = threadIdx.x, warp = tid >> 5;
     const unsigned long long deadline = globaltimer() + p.timeout_ns;
     Owner w{p, o, sh};
-    w.lo = blockIdx.x * o.block;
+    w.lo = o.rank * o.block;
     w.cnt = min(o.block, (unsigned)p.n - min(w.lo, (unsigned)p.n));
     w.out = owner_smem;
     w.in = w.out + OWNER_OUT;
@@ -590,20 +591,20 @@ __device__ __forceinline__ void owner_solve(const PlainParams &p, const OwnerPar
         sh.exit = sh.near_over = sh.range = 0u;
         sh.pushed = sh.relaxed = sh.sent = 0ull;
     }
-    if (blockIdx.x == 0) {
+    if (o.rank == 0) {
         for (int i = (int)tid; i < ctl::WORDS; i += OWNER_THREADS)
             if (i != ctl::BAR_COUNT && i != ctl::BAR_GEN) p.ctlw[i] = 0u;
         // The source is the first message, to its owner's inbox.
         const unsigned c = (unsigned)p.src / o.block;
-        for (unsigned i = tid; i < gridDim.x; i += OWNER_THREADS) o.tails[32u * i] = i == c;
+        for (unsigned i = tid; i < o.size; i += OWNER_THREADS) o.tails[32u * i] = i == c;
         if (tid == 0) p.l2[(size_t)c << o.inbox_log] = rec_pack((unsigned)p.src, 0u, 0u);
     }
-    if (!grid_barrier(p.ctlw, gridDim.x, deadline)) return;
+    if (!grid_barrier(p.ctlw, o.size, deadline)) return;
 
     if (warp < OWNER_WORKERS) owner_work<Arcs, LPV>(w, deadline);
     else if (warp == OWNER_WORKERS) owner_sender(p, o, sh, w.out, deadline);
     else if (warp == OWNER_WORKERS + 1) owner_receiver(p, o, sh, w.in);
-    else if (blockIdx.x == 0) owner_controller(p, o, deadline);
+    else if (o.rank == 0) owner_controller(p, o, deadline);
 
     __syncthreads();
     for (unsigned i = tid; i < w.cnt; i += OWNER_THREADS) p.dist[w.lo + i] = w.dist[i];

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 #include <cstddef>
+#include <cstdint>
 
 namespace mlmq {
 
@@ -37,6 +38,9 @@ cudaError_t plain_launch(const PlainParams &p, int unroll, int grid, cudaStream_
 int owner_threads();
 int owner_block(int n, int sms, int *ctas);
 size_t owner_tails_bytes(int ctas);
+// Whether a graph's shape suits the kernel with `ctas` CTAs and inboxes in
+// `rings` rings of 2^l2_log slots; `away` as mlmq_graph::away.
+int owner_fits(int n, int64_t m, int max_degree, float away, int ctas, int rings, int l2_log);
 cudaError_t owner_prepare();
 cudaError_t owner_launch(const PlainParams &p, int block, int ctas, unsigned *tails,
                          cudaStream_t stream);

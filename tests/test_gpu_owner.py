@@ -90,3 +90,28 @@ def test_sums_beyond_the_range_are_reported(first, second):
     del ei
     assert np.array_equal(s.solve(second + 1).dist(), oracle_lib.sssp_i32(g, second + 1)[0])
     assert _owned(s)
+
+
+@pytest.mark.parametrize("n,deg,reach,wmax", [(31, 2, 5, 9), (16384, 24, 8000, 50),
+                                              (16385, 8, 300, 10**6), (70001, 9, 1500, 10**5)])
+def test_noalloc_in_place(n, deg, reach, wmax):
+    """The caller's CSR read in place, in a local order and shuffled (the
+    asynchronous kernel), on the one workspace in turn."""
+    import ctypes
+    import torch
+    from mlmq_tpds_withl3_b200 import default_config
+    from mlmq_tpds_withl3_b200._lib import check, lib
+    g = _band(n, deg, reach, wmax, n)
+    perm = np.random.default_rng(2).permutation(n)
+    mixed = _csr(n, perm[np.repeat(np.arange(n), np.diff(g.row))], perm[g.col], g.w, "shuffled")
+    out = torch.empty(n, dtype=torch.int32, device="cuda")
+    cfg = default_config()
+    ref, _ = oracle_lib.sssp_i32(g, n // 3)
+    for h, src, back in ((g, n // 3, None), (mixed, int(perm[n // 3]), perm)) * 2:
+        row, col, w = (torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (h.row, h.col, h.w))
+        out.fill_(-1)
+        torch.cuda.synchronize()
+        check(lib.mlmq_sssp_solve_noalloc(n, h.m, row.data_ptr(), col.data_ptr(), w.data_ptr(), src,
+                                          out.data_ptr(), ctypes.byref(cfg), None), "noalloc")
+        got = out.cpu().numpy()
+        assert np.array_equal(got if back is None else got[back], ref)
