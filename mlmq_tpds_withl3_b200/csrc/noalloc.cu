@@ -33,6 +33,7 @@
 //    the set-up instead of trusting what it found before.
 #include "mlmq_b200.h"
 #include "solver_internal.h"
+#include "sssp_owner.h"
 #include "sssp_plain.h"
 #include "sssp_plain_body.cuh"
 

@@ -7,6 +7,7 @@
 #include <cub/device/device_segmented_sort.cuh>
 #include "mlmq_b200.h"
 #include "mlmq_queue.cuh"
+#include "sssp_owner.h"
 #include "sssp_plain.h"
 #include "solver_internal.h"
 

@@ -13,16 +13,23 @@
 // independent chains, which is where the batched throughput comes from.
 // Queries on the same graph read the same CSR, so its lines are shared in L2.
 //
-// The launch (parameter upload, kernel, status download) can be captured in
+// Queries that suit the vertex-owner kernel (sssp_owner.cuh) and fit on the GPU
+// at once or nearly so are solved by it instead, in a launch of their own
+// before this one: a query takes a third of the time there, but whole SMs, so
+// it pays while there are SMs for all of them (see plan_owner).
+//
+// The launch (parameter upload, kernels, status download) can be captured in
 // a CUDA graph and replayed (mlmq_batch_run with use_graph = 1).
 #include "mlmq_b200.h"
 #include "solver_internal.h"
+#include "sssp_owner.h"
 #include "sssp_plain.h"
 // Per-warp counters in shared memory (see mlmq_queue.cuh).
 #define MLMQ_WARP_STATS_SMEM 1
 #include "sssp_plain_body.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <new>
@@ -41,6 +48,7 @@ struct BatchQuery {
     const int4 *tiles;
     const int *split;
     int n, nslots, nids, src;
+    int slot;  // whose arrays and control block it uses
 };
 struct BatchParams {
     PlainParams base;  // configuration; dist/l2/l3/l3bits/ctlw point at slot 0's arrays
@@ -74,11 +82,11 @@ __global__ void __maxnreg__(SLOT_KERNEL_REGS) sssp_batch_kernel(BatchParams bp) 
         p.nids = qy.nids;
         p.split = qy.split;
         p.src = qy.src;
-        p.dist = bp.base.dist + s * bp.dist_stride;
-        p.l2 = bp.base.l2 + s * bp.l2_stride;
-        p.l3 = bp.base.l3 + s * bp.l3_stride;
-        p.l3bits = bp.base.l3bits + s * bp.bits_stride;
-        p.ctlw = bp.base.ctlw + s * bp.ctl_stride;
+        p.dist = bp.base.dist + qy.slot * bp.dist_stride;
+        p.l2 = bp.base.l2 + qy.slot * bp.l2_stride;
+        p.l3 = bp.base.l3 + qy.slot * bp.l3_stride;
+        p.l3bits = bp.base.l3bits + qy.slot * bp.bits_stride;
+        p.ctlw = bp.base.ctlw + qy.slot * bp.ctl_stride;
         cta_params = p;
     }
     __syncthreads();
@@ -110,6 +118,17 @@ struct mlmq_batch {
     unsigned *d_ctl = nullptr;        // max_q * CTL_STRIDE
     BatchQuery *d_queries = nullptr;  // max_q
     BatchQuery *h_queries = nullptr;  // pinned
+    // The vertex-owner part of the current query set: its queries in the order
+    // of their groups, and one plan entry per CTA.
+    struct OwnerTables {
+        OwnerQuery *queries = nullptr;  // max_q
+        OwnerCta *plan = nullptr;       // sms
+    } d_owner, h_owner;                 // device, pinned
+    unsigned *d_tails = nullptr;        // a line per CTA
+    int sms = 0, owner_nq = 0, owner_ctas = 0;
+    bool owner_wide = false, use_owner = true;
+    std::vector<int> srcs;              // of the last launch, with `held`
+    cudaStream_t last = nullptr;
     unsigned *h_ctl = nullptr;        // pinned copy of the control blocks
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;
@@ -145,8 +164,18 @@ int reset_all(mlmq_batch *b, cudaStream_t st) {
 int enqueue(mlmq_batch *b, int nq, cudaStream_t st) {
     const int threads = 32 * (b->workers + 1);
     const size_t smem = plain_smem_bytes(b->workers);
-    int rc = cuda_fail(cudaMemcpyAsync(b->d_queries, b->h_queries, sizeof(BatchQuery) * nq,
+    const int rest = nq - b->owner_nq;  // queries of the asynchronous kernel
+    int rc = MLMQ_OK;
+    if (rest)
+        rc = cuda_fail(cudaMemcpyAsync(b->d_queries, b->h_queries, sizeof(BatchQuery) * rest,
                                        cudaMemcpyHostToDevice, st), "batch queries");
+    if (!rc && b->owner_nq)
+        rc = cuda_fail(cudaMemcpyAsync(b->d_owner.queries, b->h_owner.queries,
+                                       sizeof(OwnerQuery) * b->owner_nq, cudaMemcpyHostToDevice, st),
+                       "batch owner queries");
+    if (!rc && b->owner_nq)
+        rc = cuda_fail(cudaMemcpyAsync(b->d_owner.plan, b->h_owner.plan, sizeof(OwnerCta) * b->owner_ctas,
+                                       cudaMemcpyHostToDevice, st), "batch owner plan");
     if (rc) return rc;
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)b->grid);
@@ -192,13 +221,87 @@ int enqueue(mlmq_batch *b, int nq, cudaStream_t st) {
     bp.l3_stride = (size_t)1 << b->l3_log;
     bp.bits_stride = b->bits_words;
     bp.ctl_stride = CTL_STRIDE;
-    bp.nq = nq;
+    bp.nq = rest;
+    if (b->owner_nq)
+        rc = cuda_fail(owner_batch_launch(p, bp.dist_stride, bp.l2_stride, bp.ctl_stride, b->d_owner.queries,
+                                          b->d_owner.plan, b->owner_ctas, b->owner_wide, b->d_tails,
+                                          b->graph_cooperative, st),
+                       "batch owner launch");
     void *args[] = {&bp};
-    rc = cuda_fail(cudaLaunchKernelExC(&lc, batch_kernel(b->cfg.relax_unroll, b->split), args),
-                   "batch launch");
+    if (!rc && rest)
+        rc = cuda_fail(cudaLaunchKernelExC(&lc, batch_kernel(b->cfg.relax_unroll, b->split), args),
+                       "batch launch");
     if (rc) return rc;
     return cuda_fail(cudaMemcpyAsync(b->h_ctl, b->d_ctl, sizeof(unsigned) * CTL_STRIDE * nq,
                                      cudaMemcpyDeviceToHost, st), "batch status");
+}
+
+// Lays `queries` (indexes into the launch) out on the SMs for the vertex-owner
+// kernel with blocks of at most `block` vertices: groups of CTAs, the largest
+// query first, each in a group of its own while SMs are left, then in the group
+// that has least to do.  Returns the longest group's time over the longest
+// query's, in the unit sqrt(n): a road-like query's time goes with the length of
+// its paths (1000x900 grid 3.0 ms, 512^2 1.4, 256^2 0.68).
+struct OwnerGroup {
+    int ctas;
+    double load;
+    std::vector<int> queries;
+};
+double lay_out(const mlmq_batch *b, const mlmq_graph *const *graphs, const std::vector<int> &queries,
+               int block, std::vector<OwnerGroup> &groups) {
+    groups.clear();
+    int left = b->cfg.work_blocks > 0 ? std::min(b->cfg.work_blocks, b->sms) : b->sms;
+    double longest = 0.0, most = 0.0;
+    for (int q : queries) {
+        const int ctas = (graphs[q]->n + block - 1) / block;
+        const double load = std::sqrt((double)graphs[q]->n);
+        OwnerGroup *to = nullptr;
+        if (ctas <= left) {
+            left -= ctas;
+            groups.push_back(OwnerGroup{ctas, 0.0, {}});
+            to = &groups.back();
+        } else {
+            for (OwnerGroup &g : groups)
+                if (g.ctas >= ctas && (!to || g.load < to->load)) to = &g;
+        }
+        if (!to) return HUGE_VAL;
+        to->load += load;
+        to->queries.push_back(q);
+        most = std::max(most, load);
+        longest = std::max(longest, to->load);
+    }
+    return most > 0.0 ? longest / most : HUGE_VAL;
+}
+
+// The queries of this launch for the vertex-owner kernel: those whose graph
+// suits it, when they fit side by side, or two deep.  One solve there takes
+// 0.33 to 0.45 of its time here with few others beside it (1000x900 grid 2.98
+// against 7.6 ms at 8 queries, 512^2 1.43 against 3.9, kNN 100k 0.85 against
+// 2.0) and the launch here grows only slowly with the queries (512^2 at 64:
+// 6.5 ms), so two solves in turn still win and three no longer do.  The smallest
+// blocks that fit at once are taken.
+bool plan_owner(mlmq_batch *b, int nq, const mlmq_graph *const *graphs, std::vector<OwnerGroup> &groups,
+                int *block_out) try {
+    const mlmq_config &c = b->cfg;
+    if (!b->use_owner || c.queue_type != MLMQ_L1SLF_L2DQ || c.light_heavy || c.bucket_sync) return false;
+    const int largest = owner_max_block();
+    std::vector<int> fit;
+    for (int q = 0; q < nq; q++) {
+        const mlmq_graph *g = graphs[q];
+        const int ctas = (g->n + largest - 1) / largest;
+        if (owner_fits(g->n, g->m, g->max_degree, g->away, ctas, c.bucket_num + 1, b->l2_log)) fit.push_back(q);
+    }
+    if (fit.empty()) return false;
+    std::stable_sort(fit.begin(), fit.end(), [&](int x, int y) { return graphs[x]->n > graphs[y]->n; });
+    for (int block = largest / 3 / 32 * 32;; block += largest / 6 / 32 * 32) {
+        if (block > largest) block = largest;
+        const double depth = lay_out(b, graphs, fit, block, groups);
+        *block_out = block;
+        if (depth <= 1.0) return true;
+        if (block == largest) return depth <= 2.0;
+    }
+} catch (const std::bad_alloc &) {
+    return false;
 }
 
 }  // namespace
@@ -263,6 +366,13 @@ extern "C" int mlmq_batch_create(int max_queries, int max_vertices, const mlmq_c
     if (!rc) rc = dev_alloc(&b->d_l3bits, sizeof(unsigned) * b->bits_words * nq, b->stream, "batch L3 bits");
     if (!rc) rc = dev_alloc(&b->d_ctl, sizeof(unsigned) * CTL_STRIDE * nq, b->stream, "batch ctl");
     if (!rc) rc = dev_alloc(&b->d_queries, sizeof(BatchQuery) * nq, b->stream, "batch queries");
+    b->sms = sms;
+    if (!rc) rc = dev_alloc(&b->d_owner.queries, sizeof(OwnerQuery) * nq, b->stream, "batch owner queries");
+    if (!rc) rc = dev_alloc(&b->d_owner.plan, sizeof(OwnerCta) * (size_t)sms, b->stream, "batch owner plan");
+    if (!rc) rc = dev_alloc(&b->d_tails, owner_tails_bytes(sms), b->stream, "batch owner tails");
+    if (!rc) rc = pinned_alloc(&b->h_owner.queries, sizeof(OwnerQuery) * nq);
+    if (!rc) rc = pinned_alloc(&b->h_owner.plan, sizeof(OwnerCta) * (size_t)sms);
+    if (!rc) rc = cuda_fail(owner_prepare(), "owner shared memory");
     if (!rc) rc = pinned_alloc(&b->h_queries, sizeof(BatchQuery) * nq);
     if (!rc) rc = pinned_alloc(&b->h_ctl, sizeof(unsigned) * CTL_STRIDE * nq);
     if (!rc) rc = reset_all(b, b->stream);
@@ -311,18 +421,36 @@ extern "C" int mlmq_batch_run(mlmq_batch *b, int nq, const mlmq_graph *const *gr
     for (const mlmq_graph *g : hold) graph_retain(g);
     for (const mlmq_graph *g : b->held) graph_release(g);
     b->held.swap(hold);
+    b->srcs.assign(srcs, srcs + nq);
+    b->last = st;
+    std::vector<OwnerGroup> groups;
+    int block = 0;
+    if (!plan_owner(b, nq, graphs, groups, &block)) groups.clear();
+    std::vector<char> owned((size_t)nq, 0);
+    for (const OwnerGroup &g : groups)
+        for (int q : g.queries) owned[(size_t)q] = 1;
     std::vector<long long> key;
     key.reserve(2 * (size_t)nq + 1);
     // The kernel variant is part of a captured launch: the split-capable one
-    // when a graph has pieces or the light/heavy split is on.
+    // when a graph has pieces or the light/heavy split is on.  (Which queries
+    // go to the vertex-owner kernel follows from the query set.)
     b->split = b->cfg.light_heavy != 0;
-    for (int q = 0; q < nq; q++)
+    // 64-byte tiles where a vertex has more arcs than the 32-byte ones hold.
+    b->owner_wide = b->cfg.vertex_tiles == 2;
+    for (int q = 0; q < nq; q++) {
         if (graphs[q]->pieces > 0) b->split = true;
+        if (owned[(size_t)q] && b->cfg.vertex_tiles && graphs[q]->max_degree > TILE_ARCS) b->owner_wide = true;
+    }
     key.push_back(b->split ? 1 : 0);
     b->n_of.assign((size_t)nq, 0);
+    int rest = 0;
     for (int q = 0; q < nq; q++) {
         const mlmq_graph *g = graphs[q];
-        BatchQuery &qy = b->h_queries[q];
+        b->n_of[q] = g->n;
+        key.push_back((long long)(uintptr_t)g);
+        key.push_back(srcs[q]);
+        if (owned[(size_t)q]) continue;
+        BatchQuery &qy = b->h_queries[rest++];
         qy.row = g->d_row;
         qy.arcs = g->d_arcs;
         int stride = 2;
@@ -333,9 +461,29 @@ extern "C" int mlmq_batch_run(mlmq_batch *b, int nq, const mlmq_graph *const *gr
         qy.split = nullptr;
         if (b->cfg.light_heavy && (rc = graph_light_split(g, b->cfg.delta, &qy.split))) return rc;
         qy.src = srcs[q];
-        b->n_of[q] = g->n;
-        key.push_back((long long)(uintptr_t)g);
-        key.push_back(srcs[q]);
+        qy.slot = q;
+    }
+    b->owner_nq = b->owner_ctas = 0;
+    for (const OwnerGroup &group : groups) {
+        const OwnerCta cta{b->owner_ctas, b->owner_nq, (int)group.queries.size(), 0};
+        for (int i = 0; i < group.ctas; i++) b->h_owner.plan[b->owner_ctas++] = cta;
+        for (int q : group.queries) {
+            const mlmq_graph *g = graphs[q];
+            OwnerQuery &qy = b->h_owner.queries[b->owner_nq++];
+            qy.row = g->d_row;
+            qy.arcs = g->d_arcs;
+            int stride = 2;
+            const int tiles = b->cfg.vertex_tiles == 0 ? 0 : b->owner_wide ? 2 : 1;
+            if ((rc = graph_tiles(g, tiles, &qy.tiles, &stride))) return rc;
+            qy.n = g->n;
+            qy.src = srcs[q];
+            qy.slot = q;
+            qy.size = (g->n + block - 1) / block;
+            qy.block = (unsigned)((g->n + qy.size - 1) / qy.size + 31) / 32 * 32;
+            qy.size = (int)(((unsigned)g->n + qy.block - 1) / qy.block);
+            qy.block_inv = 0xffffffffu / qy.block;
+            qy.inbox_log = owner_inbox_log(qy.size, b->cfg.bucket_num + 1, b->l2_log);
+        }
     }
     b->nq = nq;
     if (use_graph) {
@@ -389,10 +537,23 @@ extern "C" int mlmq_batch_wait(mlmq_batch *b) {
         return rc;
     }
     int worst = MLMQ_OK;
+    bool full = false;
     for (int q = 0; q < b->nq; q++) {
         const int e = status_to_error(b->h_ctl[(size_t)q * CTL_STRIDE + ctl::STATUS]);
         if (e != MLMQ_OK && e != MLMQ_ERR_RANGE) b->dirty = true;
         if (e != MLMQ_OK && worst == MLMQ_OK) worst = e;
+        full = full || e == MLMQ_ERR_QUEUE_FULL;
+    }
+    if (full && b->owner_nq) {
+        // Inboxes that filled each other up: the asynchronous kernel, whose
+        // rings divert to L3, takes this batch's queries from here on.
+        b->use_owner = false;
+        if (b->exec) cudaGraphExecDestroy(b->exec);
+        b->exec = nullptr;
+        const std::vector<const mlmq_graph *> graphs = b->held;
+        const std::vector<int> srcs = b->srcs;
+        rc = mlmq_batch_run(b, (int)graphs.size(), graphs.data(), srcs.data(), 0, b->last);
+        return rc ? rc : mlmq_batch_wait(b);
     }
     return worst;
 }
@@ -452,6 +613,11 @@ extern "C" void mlmq_batch_destroy(mlmq_batch *b) {
     dev_free(b->d_l3bits, b->stream);
     dev_free(b->d_ctl, b->stream);
     dev_free(b->d_queries, b->stream);
+    dev_free(b->d_owner.queries, b->stream);
+    dev_free(b->d_owner.plan, b->stream);
+    dev_free(b->d_tails, b->stream);
+    pinned_free(b->h_owner.queries, sizeof(OwnerQuery) * (size_t)b->max_q);
+    pinned_free(b->h_owner.plan, sizeof(OwnerCta) * (size_t)b->sms);
     pinned_free(b->h_queries, sizeof(BatchQuery) * nq);
     pinned_free(b->h_ctl, sizeof(unsigned) * CTL_STRIDE * nq);
     for (const mlmq_graph *g : b->held) graph_release(g);

@@ -1,6 +1,6 @@
 // sssp_owner.cu -- the vertex-owner kernel and its launch helpers.
 #include "sssp_owner.cuh"
-#include "sssp_plain.h"
+#include "sssp_owner.h"
 
 #include <algorithm>
 
@@ -8,13 +8,69 @@ namespace mlmq {
 
 // LPV lanes per vertex: 2 for 32-byte tiles and row offsets, 4 for 64-byte tiles.
 template <class Arcs, int LPV>
-__global__ void __launch_bounds__(OWNER_THREADS, 1) sssp_owner_kernel(PlainParams p, OwnerParams o) {
-    o.rank = blockIdx.x;
-    o.size = gridDim.x;
-    owner_solve<Arcs, LPV>(p, o);
+__global__ void __launch_bounds__(OWNER_THREADS, 1) sssp_owner_kernel(const __grid_constant__ PlainParams p,
+                                                                       const __grid_constant__ OwnerParams o) {
+    owner_solve<Arcs, LPV>(p, o, blockIdx.x, gridDim.x);
+}
+
+struct OwnerBatchParams {
+    PlainParams base;  // configuration; dist/l2/ctlw point at slot 0's arrays
+    size_t dist_stride, l2_stride, ctl_stride;
+    const OwnerQuery *__restrict__ queries;
+    const OwnerCta *__restrict__ plan;
+    unsigned *tails;
+};
+
+// Groups of CTAs that each solve their queries one after another.  A query may
+// need fewer CTAs than its group has; the others go on to the next one and
+// wait at its first barrier.
+template <int LPV>
+__global__ void __launch_bounds__(OWNER_THREADS, 1) sssp_owner_batch_kernel(const __grid_constant__ OwnerBatchParams bp) {
+    __shared__ PlainParams p;
+    __shared__ OwnerParams o;
+    const OwnerCta cta = bp.plan[blockIdx.x];
+    for (int k = 0; k < cta.count; k++) {
+        const OwnerQuery &qy = bp.queries[cta.query + k];
+        const unsigned rank = blockIdx.x - (unsigned)cta.first;
+        if (rank >= (unsigned)qy.size) continue;
+        __syncthreads();  // the query before is done with p, o and the solve's shared memory
+        if (threadIdx.x == 0) {
+            p = bp.base;
+            p.row = qy.row;
+            p.arcs = qy.arcs;
+            p.tiles = qy.tiles;
+            p.n = p.nslots = p.nids = qy.n;
+            p.src = qy.src;
+            p.dist = bp.base.dist + qy.slot * bp.dist_stride;
+            p.l2 = bp.base.l2 + qy.slot * bp.l2_stride;
+            p.ctlw = bp.base.ctlw + qy.slot * bp.ctl_stride;
+            o.block = qy.block;
+            o.block_inv = qy.block_inv;
+            o.inbox_log = qy.inbox_log;
+            o.tails = bp.tails + 32 * (size_t)cta.first;
+        }
+        __syncthreads();
+        owner_solve<ArcsInterleaved, LPV>(p, o, rank, (unsigned)qy.size);
+    }
 }
 
 namespace {
+// The CTAs of a solve wait on one another, so all of them have to be resident.
+cudaError_t launch(const void *kernel, int ctas, size_t smem, void **args, bool cooperative,
+                   cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(OWNER_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cooperative ? 1 : 0;
+    return cudaLaunchKernelExC(&cfg, kernel, args);
+}
+
 // The caller's separate arrays (no arc array) are read in place.
 const void *owner_kernel(int tile_stride, bool in_place) {
     if (in_place) return (const void *)sssp_owner_kernel<ArcsSplit, 2>;
@@ -22,16 +78,18 @@ const void *owner_kernel(int tile_stride, bool in_place) {
                             : (const void *)sssp_owner_kernel<ArcsInterleaved, 2>;
 }
 
+}  // namespace
+
 // log2 slots of each of `ctas` inboxes in the memory of the L2 rings.
-int inbox_log(int ctas, int rings, int l2_log) {
+int owner_inbox_log(int ctas, int rings, int l2_log) {
     const size_t slots = (size_t)rings << l2_log;
     int log = 0;
     while (log < 20 && ((size_t)ctas << (log + 1)) <= slots) log++;
     return log;
 }
-}  // namespace
 
 int owner_threads() { return OWNER_THREADS; }
+int owner_max_block() { return OWNER_MAX_BLOCK; }
 
 // Blocks of OWNER_BLOCK vertices while there are SMs for them, then larger
 // ones.  Smaller blocks mean shorter lists but more messages: grid 1200x777 2.9
@@ -59,7 +117,7 @@ int owner_fits(int n, int64_t m, int max_degree, float away, int ctas, int rings
     if (n > OWNER_MAX_N || max_degree > OWNER_MAX_DEGREE) return 0;
     if (ctas == 1) return 1;
     return away <= 0.125f &&
-           4.0 * (double)away * (double)m / ctas + 1024.0 <= (double)(1 << inbox_log(ctas, rings, l2_log));
+           4.0 * (double)away * (double)m / ctas + 1024.0 <= (double)(1 << owner_inbox_log(ctas, rings, l2_log));
 }
 
 cudaError_t owner_prepare() {
@@ -68,6 +126,11 @@ cudaError_t owner_prepare() {
             cudaFuncSetAttribute(owner_kernel(k == 1 ? 4 : 2, k == 2),
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)owner_smem_bytes(OWNER_MAX_BLOCK));
+        if (e != cudaSuccess) return e;
+    }
+    for (const void *k : {(const void *)sssp_owner_batch_kernel<2>, (const void *)sssp_owner_batch_kernel<4>}) {
+        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)owner_smem_bytes(OWNER_MAX_BLOCK));
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -81,21 +144,29 @@ cudaError_t owner_launch(const PlainParams &p, int block, int ctas, unsigned *ta
     o.tails = tails;
     // The inboxes share the memory of the L2 rings, which both kernels leave
     // empty.
-    o.inbox_log = inbox_log(ctas, p.nb + 1, p.l2_log);
-    o.rank = 0;
-    o.size = (unsigned)ctas;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3(OWNER_THREADS);
-    cfg.dynamicSmemBytes = owner_smem_bytes((unsigned)block);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    o.inbox_log = owner_inbox_log(ctas, p.nb + 1, p.l2_log);
     void *args[] = {const_cast<PlainParams *>(&p), &o};
-    return cudaLaunchKernelExC(&cfg, owner_kernel(p.tile_stride, p.col != nullptr), args);
+    return launch(owner_kernel(p.tile_stride, p.col != nullptr), ctas,
+                  owner_smem_bytes((unsigned)block), args, true, stream);
+}
+
+cudaError_t owner_batch_launch(const PlainParams &base, size_t dist_stride, size_t l2_stride,
+                               size_t ctl_stride, const OwnerQuery *queries, const OwnerCta *plan,
+                               int ctas, bool wide, unsigned *tails, bool cooperative,
+                               cudaStream_t stream) {
+    OwnerBatchParams bp;
+    bp.base = base;
+    bp.base.tile_stride = wide ? 4 : 2;
+    bp.base.split = nullptr;
+    bp.dist_stride = dist_stride;
+    bp.l2_stride = l2_stride;
+    bp.ctl_stride = ctl_stride;
+    bp.queries = queries;
+    bp.plan = plan;
+    bp.tails = tails;
+    void *args[] = {&bp};
+    return launch(wide ? (const void *)sssp_owner_batch_kernel<4> : (const void *)sssp_owner_batch_kernel<2>,
+                  ctas, owner_smem_bytes(OWNER_MAX_BLOCK), args, cooperative, stream);
 }
 
 }  // namespace mlmq

@@ -71,7 +71,6 @@ struct OwnerParams {
     unsigned block, block_inv;  // vertices per CTA (a multiple of 32), (2^32 - 1) / block
     int inbox_log;              // log2 slots of one inbox ring
     unsigned *tails;            // [CTAs] one 128-byte line each
-    unsigned rank, size;        // this CTA among the solve's
 };
 
 // Shared memory: distances, near bits, far bits, near lists, far lists.
@@ -96,7 +95,7 @@ struct OwnerShared {
     unsigned least[2];    // smallest far distance, by tick parity
     unsigned near_over;   // near bits without a list entry exist
     unsigned range;
-    unsigned long long pushed, relaxed, sent;
+    unsigned long long pushed, relaxed, sent, busy;
 };
 
 __device__ __forceinline__ void owner_bar() {
@@ -117,6 +116,7 @@ struct Owner {
     const PlainParams &p;
     const OwnerParams &o;
     OwnerShared &sh;
+    unsigned rank, size;  // this CTA among the solve's
     unsigned lo, cnt;     // first vertex and vertices of the block
     int *dist;
     unsigned *near_bits, *far_bits;
@@ -126,6 +126,7 @@ struct Owner {
     unsigned next_slot;   // near_n index and list half that pushes go to
     unsigned next_half, far_half;
     unsigned pushed, relaxed, sent;
+    unsigned busy;        // ticks that relaxed something (the clerk)
     bool range;
 };
 
@@ -397,6 +398,7 @@ __device__ __forceinline__ void owner_work(Owner &w, unsigned long long deadline
         for (unsigned i0 = (tid >> 5) * (32u / LPV); i0 < n; i0 += OWNER_T / LPV)
             owner_relax<Arcs, LPV>(w, list, i0, n, deadline);
         ticks += n != 0u;
+        w.busy += clerk && n != 0u;
         owner_bar();
         slot = w.next_slot;
         head = ld_shared4(&sh.tick[slot]);
@@ -497,9 +499,9 @@ __device__ __forceinline__ void owner_sender(const PlainParams &p, const OwnerPa
 // The receiver warp: this CTA's inbox ring to the shared-memory inbox; it also
 // brings the end of the solve to the CTA.
 __device__ __forceinline__ void owner_receiver(const PlainParams &p, const OwnerParams &o,
-                                               OwnerShared &sh, unsigned long long *in) {
+                                               OwnerShared &sh, unsigned long long *in, unsigned rank) {
     const unsigned lane = threadIdx.x & 31u;
-    unsigned long long *ring = p.l2 + ((size_t)o.rank << o.inbox_log);
+    unsigned long long *ring = p.l2 + ((size_t)rank << o.inbox_log);
     const unsigned mask = (1u << o.inbox_log) - 1u;
     unsigned at = 0;
     for (;;) {
@@ -532,7 +534,7 @@ __device__ __forceinline__ void owner_receiver(const PlainParams &p, const Owner
 
 // CTA 0's controller warp: the end of the solve and the time limit.
 __device__ __forceinline__ void owner_controller(const PlainParams &p, const OwnerParams &o,
-                                                 unsigned long long deadline) {
+                                                 unsigned size, unsigned long long deadline) {
     const unsigned lane = threadIdx.x & 31u;
     for (;;) {
         // CREDIT before the tails: a credit is returned only after the sends
@@ -541,7 +543,7 @@ __device__ __forceinline__ void owner_controller(const PlainParams &p, const Own
         const unsigned credit = ld_acquire(p.ctlw + ctl::CREDIT);
         __syncwarp();
         unsigned sum = 0;
-        for (unsigned c = lane; c < o.size; c += 32) sum += ld_relaxed(o.tails + 32u * c);
+        for (unsigned c = lane; c < size; c += 32) sum += ld_relaxed(o.tails + 32u * c);
         sum = __reduce_add_sync(FULL, sum);
         if (sum == __shfl_sync(FULL, credit, 0)) {
             if (lane == 0) {
@@ -558,14 +560,16 @@ __device__ __forceinline__ void owner_controller(const PlainParams &p, const Own
     }
 }
 
+// The solve, by CTA `rank` of its `size`, all of them resident.
 template <class Arcs, int LPV>
-__device__ __forceinline__ void owner_solve(const PlainParams &p, const OwnerParams &o) {
+__device__ __forceinline__ void owner_solve(const PlainParams &p, const OwnerParams &o, unsigned rank,
+                                            unsigned size) {
     extern __shared__ unsigned long long owner_smem[];
     __shared__ OwnerShared sh;
     const unsigned tid = threadIdx.x, warp = tid >> 5;
     const unsigned long long deadline = globaltimer() + p.timeout_ns;
-    Owner w{p, o, sh};
-    w.lo = o.rank * o.block;
+    Owner w{p, o, sh, rank, size};
+    w.lo = w.rank * o.block;
     w.cnt = min(o.block, (unsigned)p.n - min(w.lo, (unsigned)p.n));
     w.out = owner_smem;
     w.in = w.out + OWNER_OUT;
@@ -575,7 +579,7 @@ __device__ __forceinline__ void owner_solve(const PlainParams &p, const OwnerPar
     w.near_list = w.far_bits + o.block / 32u;
     w.far_list = w.near_list + 2 * OWNER_NEAR;
     w.next_slot = w.next_half = w.far_half = 0u;
-    w.pushed = w.relaxed = w.sent = 0u;
+    w.pushed = w.relaxed = w.sent = w.busy = 0u;
     w.range = false;
     // The first bucket is a fraction of the configured width, which is the
     // most that later ones may grow to.
@@ -589,33 +593,35 @@ __device__ __forceinline__ void owner_solve(const PlainParams &p, const OwnerPar
         sh.far_n[0] = sh.far_n[1] = 0u;
         sh.in_tail = sh.in_head = sh.out_tail = sh.out_sent = 0u;
         sh.exit = sh.near_over = sh.range = 0u;
-        sh.pushed = sh.relaxed = sh.sent = 0ull;
+        sh.pushed = sh.relaxed = sh.sent = sh.busy = 0ull;
     }
-    if (o.rank == 0) {
+    if (w.rank == 0) {
         for (int i = (int)tid; i < ctl::WORDS; i += OWNER_THREADS)
             if (i != ctl::BAR_COUNT && i != ctl::BAR_GEN) p.ctlw[i] = 0u;
         // The source is the first message, to its owner's inbox.
         const unsigned c = (unsigned)p.src / o.block;
-        for (unsigned i = tid; i < o.size; i += OWNER_THREADS) o.tails[32u * i] = i == c;
+        for (unsigned i = tid; i < w.size; i += OWNER_THREADS) o.tails[32u * i] = i == c;
         if (tid == 0) p.l2[(size_t)c << o.inbox_log] = rec_pack((unsigned)p.src, 0u, 0u);
     }
-    if (!grid_barrier(p.ctlw, o.size, deadline)) return;
+    if (!grid_barrier(p.ctlw, w.size, deadline)) return;
 
     if (warp < OWNER_WORKERS) owner_work<Arcs, LPV>(w, deadline);
     else if (warp == OWNER_WORKERS) owner_sender(p, o, sh, w.out, deadline);
-    else if (warp == OWNER_WORKERS + 1) owner_receiver(p, o, sh, w.in);
-    else if (o.rank == 0) owner_controller(p, o, deadline);
+    else if (warp == OWNER_WORKERS + 1) owner_receiver(p, o, sh, w.in, rank);
+    else if (rank == 0) owner_controller(p, o, size, deadline);
 
     __syncthreads();
     for (unsigned i = tid; i < w.cnt; i += OWNER_THREADS) p.dist[w.lo + i] = w.dist[i];
     const unsigned pushed = __reduce_add_sync(FULL, w.pushed);
     const unsigned relaxed = __reduce_add_sync(FULL, w.relaxed);
     const unsigned sent = __reduce_add_sync(FULL, w.sent);
+    const unsigned busy = __reduce_add_sync(FULL, w.busy);
     if (w.range) sh.range = 1u;
     if ((tid & 31u) == 0) {
         atomicAdd(&sh.pushed, (unsigned long long)pushed);
         atomicAdd(&sh.relaxed, (unsigned long long)relaxed);
         atomicAdd(&sh.sent, (unsigned long long)sent);
+        atomicAdd(&sh.busy, (unsigned long long)busy);
     }
     __syncthreads();
     if (tid == 0) {
@@ -623,6 +629,7 @@ __device__ __forceinline__ void owner_solve(const PlainParams &p, const OwnerPar
         atomicAdd(st + ctl::ST_PUSHED, sh.pushed + sh.sent);
         atomicAdd(st + ctl::ST_RELAXED, sh.relaxed);
         atomicAdd(st + ctl::ST_IMPROVED, sh.pushed);
+        atomicAdd(st + ctl::ST_BATCHES, sh.busy);
         if (sh.range) atomicOr(p.ctlw + ctl::STATUS, ST_RANGE);
     }
 }

@@ -1,0 +1,52 @@
+// sssp_owner.h -- host side of the vertex-owner kernel (sssp_owner.cuh).
+#pragma once
+
+#include <cuda_runtime.h>
+#include <cstddef>
+#include <cstdint>
+
+namespace mlmq {
+
+struct PlainParams;
+
+int owner_threads();
+// Most vertices one CTA can own.
+int owner_max_block();
+// Vertices per CTA (a multiple of 32) and CTAs for n vertices of a plain solve
+// on `sms` SMs, 0 if they do not fit.
+int owner_block(int n, int sms, int *ctas);
+size_t owner_tails_bytes(int ctas);
+// Whether a graph's shape suits the kernel with `ctas` CTAs and inboxes in
+// `rings` rings of 2^l2_log slots; `away` as mlmq_graph::away.
+int owner_fits(int n, int64_t m, int max_degree, float away, int ctas, int rings, int l2_log);
+// Sets the kernels' shared-memory limit, before the first launch.
+cudaError_t owner_prepare();
+// One solve by `ctas` CTAs of `block` vertices each.
+cudaError_t owner_launch(const PlainParams &p, int block, int ctas, unsigned *tails,
+                         cudaStream_t stream);
+
+// A query of a batched launch, by CTAs [0, size) of its group.
+struct OwnerQuery {
+    const int *row;
+    const int2 *arcs;
+    const int4 *tiles;
+    int n, src, slot;
+    unsigned block, block_inv;
+    int size, inbox_log;
+};
+// What a CTA of a batched launch does: its group's first CTA, and the group's
+// queries [query, query + count), one after another.
+struct OwnerCta {
+    int first, query, count, pad;
+};
+int owner_inbox_log(int ctas, int rings, int l2_log);
+// Queries `queries` (device) by `ctas` CTAs as `plan` (device, one entry a CTA)
+// says; `base` holds the configuration and slot 0's arrays, the strides are
+// between slots (elements), `wide` tells 64-byte tiles; `cooperative` as a plain
+// launch would be: never more CTAs than SMs.
+cudaError_t owner_batch_launch(const PlainParams &base, size_t dist_stride, size_t l2_stride,
+                               size_t ctl_stride, const OwnerQuery *queries, const OwnerCta *plan,
+                               int ctas, bool wide, unsigned *tails, bool cooperative,
+                               cudaStream_t stream);
+
+}  // namespace mlmq

@@ -3,7 +3,6 @@
 
 #include <cuda_runtime.h>
 #include <cstddef>
-#include <cstdint>
 
 namespace mlmq {
 
@@ -31,18 +30,5 @@ size_t plain_smem_limit();
 cudaError_t plain_max_blocks_per_sm(int workers, int unroll, int *blocks);
 // Cooperative launch of `grid` CTAs on `stream`.
 cudaError_t plain_launch(const PlainParams &p, int unroll, int grid, cudaStream_t stream);
-
-// The vertex-owner kernel (sssp_owner.cuh).  owner_block: vertices per CTA (a
-// multiple of 32) and CTAs for n vertices, 0 if they do not fit; owner_prepare
-// sets the kernels' shared-memory limit, before the first launch.
-int owner_threads();
-int owner_block(int n, int sms, int *ctas);
-size_t owner_tails_bytes(int ctas);
-// Whether a graph's shape suits the kernel with `ctas` CTAs and inboxes in
-// `rings` rings of 2^l2_log slots; `away` as mlmq_graph::away.
-int owner_fits(int n, int64_t m, int max_degree, float away, int ctas, int rings, int l2_log);
-cudaError_t owner_prepare();
-cudaError_t owner_launch(const PlainParams &p, int block, int ctas, unsigned *tails,
-                         cudaStream_t stream);
 
 }  // namespace mlmq

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 import oracle_lib
-from mlmq_tpds_withl3_b200 import DeviceGraph, HostGraph, MlmqError, Solver
+from mlmq_tpds_withl3_b200 import BatchSolver, DeviceGraph, HostGraph, MlmqError, Solver
 from mlmq_tpds_withl3_b200._lib import MLMQ_ERR_RANGE
 
 pytestmark = pytest.mark.gpu
@@ -115,3 +115,27 @@ def test_noalloc_in_place(n, deg, reach, wmax):
                                           out.data_ptr(), ctypes.byref(cfg), None), "noalloc")
         got = out.cpu().numpy()
         assert np.array_equal(got if back is None else got[back], ref)
+
+
+def test_batches_of_owned_and_other_queries():
+    """One batch object for query sets of one to many queries: graphs of one
+    block and of several, two queries deep in their groups, beside ones for the
+    asynchronous kernel (hubs, shuffled), launched and replayed in turn."""
+    small, large = HostGraph.grid(90, 70, seed=5), HostGraph.grid(700, 800, seed=6)
+    bands, hubs = _band(50000, 7, 300, 10**5, 8), HostGraph.rmat(12, seed=9)
+    perm = np.random.default_rng(3).permutation(bands.n)
+    mixed = _csr(bands.n, perm[np.repeat(np.arange(bands.n), np.diff(bands.row))], perm[bands.col],
+                 bands.w, "shuffled")
+    hosts = [small, large, bands, hubs, mixed]
+    dgs = [DeviceGraph.upload(h) for h in hosts]
+    rng = np.random.default_rng(4)
+    sets = [[1] * 16, [0], [0] * 60, [3, 4], [0, 1, 2, 3, 4] * 5, [2] * 40 + [0] * 20]
+    b = BatchSolver(64, max(g.slots for g in dgs), {"timeout_ms": 5000})
+    for which in sets:
+        queries = [(k, int(rng.integers(hosts[k].n))) for k in which]
+        refs = [oracle_lib.sssp_i32(hosts[k], src) for k, src in queries]
+        for use_graph in (False, True, True):
+            b.run([(dgs[k], src) for k, src in queries], use_graph=use_graph)
+            for q, (ref, work) in enumerate(refs):
+                assert np.array_equal(b.dist(q), ref), (which, use_graph, q)
+                assert b.stats(q)["relaxed"] >= work and b.stats(q)["batches"] > 0
