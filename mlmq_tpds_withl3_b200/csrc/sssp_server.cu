@@ -455,11 +455,14 @@ int server_create(int slots, const int *layout, int max_vertices, const mlmq_con
     const size_t per_slot = sizeof(int) * (size_t)max_vertices +
                             8 * (((size_t)(cfg.bucket_num + 1) << sv->l2_log) + ((size_t)1 << sv->l3_log)) +
                             4 * SRV_CTL_STRIDE + 4 * sv->bits_words;
-    size_t free_b = 0, total_b = 0;
-    // Memory the library's pool keeps for reuse counts as free here.
-    if (!rc) rc = mlmq_release_cached();
+    size_t free_b = 0, total_b = 0, kept_b = 0;
+    // Memory the library's pool keeps for reuse counts as free here.  It is not
+    // handed to the driver first: unmapping and mapping a few GB took 40 to 90
+    // ms of a server's creation.
+    if (!rc) rc = pool_unused(&kept_b);
     if (!rc) rc = cuda_fail(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
     if (!rc) {
+        free_b += kept_b;
         const size_t reserve = (size_t)2 << 30;
         const size_t fit = free_b > reserve ? (free_b - reserve) / per_slot : 0;
         sv->slots = (int)std::min<size_t>((size_t)slots, fit);
