@@ -92,7 +92,8 @@ typedef struct mlmq_config {
                             directly, its returned value decides the push */
     int relax_unroll;    /* rounds of 32 arcs a warp keeps in flight: 1, 2 or
                             4 (default 4; above 1 at most
-                            MLMQ_MAX_UNROLLED_WARPS worker warps per CTA) */
+                            MLMQ_MAX_UNROLLED_WARPS worker warps per CTA;
+                            batches and servers keep at most 2) */
     int l1_ahead;        /* a winner stays in the warp's L1 only while its
                             bucket is below first + l1_ahead, else it goes
                             to L2/L3 through the warp's outbox (default 4;

@@ -93,12 +93,13 @@ __global__ void __maxnreg__(SLOT_KERNEL_REGS) sssp_batch_kernel(BatchParams bp) 
     plain_body<ArcsInterleaved, K, kSplit>(cta_params, blockIdx.x - lo, hi - lo);
 }
 
+// Two rounds of arcs in flight at most, also where four are configured: many
+// warps share an SM here, so more rounds hide little and their larger loop body
+// misses the instruction cache (32 queries on R-MAT 18 10.6 against 8.2 ms, a mix
+// of R-MAT 15, 17 and a 2000x1800 grid 29.3 against 25.1).
 const void *batch_kernel(int unroll, bool split) {
-    switch (unroll) {
-        case 1: return split ? (const void *)sssp_batch_kernel<1, true> : (const void *)sssp_batch_kernel<1, false>;
-        case 2: return split ? (const void *)sssp_batch_kernel<2, true> : (const void *)sssp_batch_kernel<2, false>;
-        default: return split ? (const void *)sssp_batch_kernel<4, true> : (const void *)sssp_batch_kernel<4, false>;
-    }
+    if (unroll == 1) return split ? (const void *)sssp_batch_kernel<1, true> : (const void *)sssp_batch_kernel<1, false>;
+    return split ? (const void *)sssp_batch_kernel<2, true> : (const void *)sssp_batch_kernel<2, false>;
 }
 
 }  // namespace mlmq

@@ -360,12 +360,10 @@ __global__ void __maxnreg__(SLOT_KERNEL_REGS) sssp_server_kernel(ServerParams sp
     }
 }
 
+// Two rounds of arcs in flight at most, as in the batched kernel: a burst of 192
+// queries on three grids and R-MAT 18 took 65.9 ms with four, 51 with two.
 const void *server_kernel(int unroll) {
-    switch (unroll) {
-        case 1: return (const void *)sssp_server_kernel<1>;
-        case 2: return (const void *)sssp_server_kernel<2>;
-        default: return (const void *)sssp_server_kernel<4>;
-    }
+    return unroll == 1 ? (const void *)sssp_server_kernel<1> : (const void *)sssp_server_kernel<2>;
 }
 
 }  // namespace
