@@ -803,28 +803,13 @@ __device__ __forceinline__ void relax_batch(const PlainParams &p, WarpQ &q, uint
     }
     if constexpr (kStatsSmem) wstat_add(WS_RELAXED, __reduce_add_sync(FULL, (unsigned)deg));
     else q.relaxed += (unsigned)deg;
-    // Whole-warp relaxation of large vertices (sssp_run.cu:192-265).
+    // Whole-warp relaxation of large vertices (sssp_run.cu:192-265), one after
+    // another, then the arcs of the others, in one loop with one copy of the
+    // relaxation and the queue code in it: two copies missed the instruction
+    // cache more (32 queries on R-MAT 18 8.4 -> 7.6 ms, R-MAT 22 alone 4.1 ->
+    // 3.9, kNN 6.3M 8.0 -> 7.75).
     unsigned big = __ballot_sync(FULL, deg >= p.large);
-    while (big) {
-        const int sl = __ffs(big) - 1;
-        big &= big - 1;
-        const int lb = __shfl_sync(FULL, beg, sl);
-        const int ld = __shfl_sync(FULL, deg, sl);
-        const unsigned lu = __shfl_sync(FULL, du, sl);
-        for (int e0 = 0; e0 < ld; e0 += 32 * K) {
-            bool ok[K];
-            int ai[K];
-            unsigned uu[K];
-#pragma unroll
-            for (int k = 0; k < K; k++) {
-                const int e = e0 + 32 * k + lane;
-                ok[k] = e < ld;
-                ai[k] = lb + e;
-                uu[k] = lu;
-            }
-            relax_rounds<Arcs, K>(p, q, ring, stage, ok, ai, uu, (ld - e0 + 31) >> 5);
-        }
-    }
+    const int lbeg = beg, ldeg = deg;
     if (deg >= p.large) deg = 0;
     // Small vertices: one arc per lane through an exclusive prefix sum of
     // degrees (sssp_run.cu:269-379); the owner lane of arc e is the last lane
@@ -837,7 +822,7 @@ __device__ __forceinline__ void relax_batch(const PlainParams &p, WarpQ &q, uint
     }
     const int total = __shfl_sync(FULL, incl, 31);
     const int off = incl - deg;
-    if (K >= 4 && total <= 32) {
+    if (K >= 4 && !big && total <= 32) {
         // One round of arcs: the other rounds' owner searches and predicated
         // loads would be wasted on the critical path of a single solve.
         // (Measured: single solves 2.5-4 % faster; in the 2-round batched
@@ -858,7 +843,7 @@ __device__ __forceinline__ void relax_batch(const PlainParams &p, WarpQ &q, uint
         }
         return;
     }
-    if (K >= 4 && total <= 64) {
+    if (K >= 4 && !big && total <= 64) {
         // Two rounds of arcs (C2: 2.35 -> 2.46 GTEPS over the one-round
         // dispatch alone).
         bool ok2[2];
@@ -882,26 +867,50 @@ __device__ __forceinline__ void relax_batch(const PlainParams &p, WarpQ &q, uint
         relax_rounds<Arcs, 2>(p, q, ring, stage, ok2, ai2, uu2, 2);
         return;
     }
-    for (int e0 = 0; e0 < total; e0 += 32 * K) {
+    int e0 = 0;
+    while (big || e0 < total) {
         bool ok[K];
         int ai[K];
         unsigned uu[K];
+        int left;
+        if (big) {
+            const int sl = __ffs(big) - 1;
+            const int lb = __shfl_sync(FULL, lbeg, sl);
+            const int ld = __shfl_sync(FULL, ldeg, sl);
+            const unsigned lu = __shfl_sync(FULL, du, sl);
 #pragma unroll
-        for (int k = 0; k < K; k++) {
-            const int e = e0 + 32 * k + lane;
-            int j = 0;
-#pragma unroll
-            for (int s = 16; s > 0; s >>= 1) {
-                const int oc = __shfl_sync(FULL, off, j + s);
-                if (oc <= e) j += s;
+            for (int k = 0; k < K; k++) {
+                const int e = e0 + 32 * k + lane;
+                ok[k] = e < ld;
+                ai[k] = lb + e;
+                uu[k] = lu;
             }
-            const int ob = __shfl_sync(FULL, beg, j);
-            const int oo = __shfl_sync(FULL, off, j);
-            uu[k] = __shfl_sync(FULL, du, j);
-            ok[k] = e < total;
-            ai[k] = ob + (e - oo);
+            left = ld - e0;
+            e0 += 32 * K;
+            if (e0 >= ld) {
+                big &= big - 1;
+                e0 = 0;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < K; k++) {
+                const int e = e0 + 32 * k + lane;
+                int j = 0;
+#pragma unroll
+                for (int s = 16; s > 0; s >>= 1) {
+                    const int oc = __shfl_sync(FULL, off, j + s);
+                    if (oc <= e) j += s;
+                }
+                const int ob = __shfl_sync(FULL, beg, j);
+                const int oo = __shfl_sync(FULL, off, j);
+                uu[k] = __shfl_sync(FULL, du, j);
+                ok[k] = e < total;
+                ai[k] = ob + (e - oo);
+            }
+            left = total - e0;
+            e0 += 32 * K;
         }
-        relax_rounds<Arcs, K>(p, q, ring, stage, ok, ai, uu, (total - e0 + 31) >> 5);
+        relax_rounds<Arcs, K>(p, q, ring, stage, ok, ai, uu, (left + 31) >> 5);
     }
 }
 
