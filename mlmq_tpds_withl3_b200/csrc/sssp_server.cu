@@ -536,6 +536,10 @@ int server_create(int slots, const int *layout, int max_vertices, const mlmq_con
     if (!rc) rc = cuda_fail(cudaMemsetAsync(sv->d_ctl, 0, 4 * ns * SRV_CTL_STRIDE, sv->kstream), "reset ctl");
     if (!rc) rc = cuda_fail(cudaMemsetAsync(sv->d_cmd, 0, sizeof(SlotCommand) * ns, sv->kstream), "reset mailboxes");
     if (!rc) rc = cuda_fail(cudaMemsetAsync(sv->d_shutdown, 0, 64, sv->kstream), "reset shutdown");
+    // Commands go over on a stream of their own: not before the resets, which
+    // would wipe a query submitted right after this returns.
+    if (!rc) rc = cuda_fail(cudaEventRecord(sv->kdone, sv->kstream), "resets event");
+    if (!rc) rc = cuda_fail(cudaStreamWaitEvent(sv->qstream, sv->kdone, 0), "commands after resets");
     if (!rc) {
         ServerParams sp{};
         PlainParams &b = sp.base;
