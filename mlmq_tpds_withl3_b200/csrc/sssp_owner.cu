@@ -107,14 +107,16 @@ size_t owner_tails_bytes(int ctas) { return 128 * (size_t)ctas; }
 
 // Vertices in a local order, none of many arcs: the wavefront then hops inside
 // an SM (with many arcs between blocks it would send messages instead, and a
-// vertex of many arcs would hold up its CTA's ticks).  Above OWNER_MAX_N
-// vertices its longer lists and tiles from HBM take as long as the asynchronous
-// kernel's hops (3M points 6.2 ms on both, 6.3M points 8.0 against 7.9).  Each
-// inbox must hold its share of the arcs between blocks several times over, so
+// vertex of many arcs would hold up its CTA's ticks).  Above a number of
+// vertices its longer lists and 64-byte tiles from HBM take as long as the
+// asynchronous kernel's hops (3M points 6.6 against 7.4 ms, 6.3M points 8.0
+// against 7.9); with the 32-byte tiles of a grid it stays ahead while the blocks
+// fit (2300^2 9.6 against 12.0 ms).  Each inbox must hold its share of the arcs between blocks several times over, so
 // that a full one is out of the question in practice.
 int owner_fits(int n, int64_t m, int max_degree, float away, int ctas, int rings, int l2_log) {
-    constexpr int OWNER_MAX_N = 3 << 20, OWNER_MAX_DEGREE = 32;
-    if (n > OWNER_MAX_N || max_degree > OWNER_MAX_DEGREE) return 0;
+    constexpr int OWNER_MAX_N = 3 << 20, OWNER_MAX_N_INLINE = 6 << 20, OWNER_MAX_DEGREE = 32;
+    if (n > (max_degree <= TILE_ARCS ? OWNER_MAX_N_INLINE : OWNER_MAX_N) || max_degree > OWNER_MAX_DEGREE)
+        return 0;
     if (ctas == 1) return 1;
     return away <= 0.125f &&
            4.0 * (double)away * (double)m / ctas + 1024.0 <= (double)(1 << owner_inbox_log(ctas, rings, l2_log));
